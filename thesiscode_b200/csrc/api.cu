@@ -1,5 +1,6 @@
 // C ABI of libthesiscode_b200: context, parameters, the one-call velocity
 // sums and the device-resident RK4 driver.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -145,10 +146,11 @@ int velocity_device(tc_ctx* ctx, int cls, const double* X, int m, const double* 
   if (rc) return rc;
   double4* src = ctx->scratch[0].as<double4>();
   int* perm = nullptr;
-  if (ctx->precision == TC_FP32C && ctx->target_order == TC_ORDER_HILBERT && i1 > i0) {
+  if (i1 > i0 && tcb::wants_order(ctx)) {
     if ((rc = ctx->scratch[4].ensure((size_t)m * sizeof(int)))) return rc;
     perm = ctx->scratch[4].as<int>();
-    if ((rc = tcb::compute_order(ctx, X, i0, i1, perm, m, m))) return rc;
+    const tcb::OrderJob job{X, i0, i1, perm, m, m};
+    if ((rc = tcb::compute_orders(ctx, &job, 1))) return rc;
   }
   const long long src_len = (long long)(ctx->scratch[0].bytes / sizeof(double4));
   if ((rc = tcb::launch_pack(ctx, src_x, vort, area, n, src, src_len))) return rc;
@@ -583,20 +585,20 @@ extern "C" int tc_rk4_stage_range(tc_ctx* ctx, int stage, double dt, int a0, int
                          first ? R.x0V.as<double>() : R.xiV.as<double>(),
                          first ? R.x0Q.as<double>() : R.xiQ.as<double>()};
   const int range[6] = {a0, a1, v0, v1, q0, q1};
-  // FP32C visiting order: computed from the stage-0 positions once per step
-  // (targets move by O(dt) within a step) and whenever the ranges change.
-  const bool want_order = ctx->precision == TC_FP32C && ctx->target_order == TC_ORDER_HILBERT;
+  // FP32C visiting order: computed from the stage-0 positions once per step (targets move by
+  // O(dt) within a step) and whenever the ranges change
+  const bool want_order = tcb::wants_order(ctx);
   if (!want_order) {
     R.ordered = false;
   } else if (first || !R.ordered || memcmp(range, R.order_range, sizeof(range)) != 0) {
     tcb::DevBuf* pb[3] = {&R.permA, &R.permV, &R.permQ};
     const int nn[3] = {R.nA, R.nV, R.nQ};
+    tcb::OrderJob jobs[3];
     for (int c = 0; c < 3; ++c) {
       if ((rc = pb[c]->ensure((size_t)std::max(nn[c], 1) * sizeof(int)))) return rc;
-      if ((rc = tcb::compute_order(ctx, tx[c], range[2 * c], range[2 * c + 1], pb[c]->as<int>(),
-                                   nn[c], nn[c])))
-        return rc;
+      jobs[c] = tcb::OrderJob{tx[c], range[2 * c], range[2 * c + 1], pb[c]->as<int>(), nn[c], nn[c]};
     }
+    if ((rc = tcb::compute_orders(ctx, jobs, 3))) return rc;
     memcpy(R.order_range, range, sizeof(range));
     R.ordered = true;
   }

@@ -166,16 +166,24 @@ int launch_pack(tc_ctx* ctx, const double* x, const double* zeta, const double* 
 int launch_velocity_epilogue(tc_ctx* ctx, const double* x, const int* perm, int m, int i0, int i1,
                              int row_offset, int n_out, int nchunks, double* dX, double* dVort,
                              const double* partial = nullptr, long long partial_len = 0);
-// perm[i0..i1) <- i0..i1-1 sorted along the cube-face Hilbert curve (sphere_order.cuh);
-// x holds x_len points, perm perm_len entries (a range past either is an error)
-int compute_order(tc_ctx* ctx, const double* x, int i0, int i1, int* perm, long long x_len,
-                  long long perm_len);
+// perm[i0..i1) <- i0..i1-1 sorted along the cube-face Hilbert curve (sphere_order.cuh), for
+// up to three classes; x holds x_len points, perm perm_len entries (a range past either is
+// an error)
+struct OrderJob {
+  const double* x;
+  int i0, i1;
+  int* perm;
+  long long x_len, perm_len;
+};
+int compute_orders(tc_ctx* ctx, const OrderJob* jobs, int count);
+// Does a call visit its targets in that order?
+bool wants_order(const tc_ctx* ctx);
 // Extents of an order computation: points in x, entries in perm, entries in each key and
 // index buffer.
 struct OrderExtents {
   long long x_len, perm_len, key_len;
 };
-// The same in caller-provided scratch (keys in/out and indices: i1 - i0 entries each; temp:
+// One order in caller-provided scratch (keys in/out and indices: i1 - i0 entries each; temp:
 // order_sort_bytes(i1 - i0) bytes); allocates nothing.
 int order_sort_bytes(int n, size_t* bytes);
 int compute_order_into(tc_ctx* ctx, const double* x, int i0, int i1, int* perm, unsigned* k_in,
