@@ -46,7 +46,7 @@ extern "C" {
                       cancellation-free denominator, FP64 accumulation of
                       per-tile FP32 partial sums                              */
 
-/* ---- visiting order of targets in the FP32C pair kernel --------------- */
+/* ---- visiting order of targets in the pair kernels ---------------------- */
 #define TC_ORDER_GIVEN 0   /* the caller's order                             */
 #define TC_ORDER_HILBERT 1 /* along a Hilbert curve over the cube faces (default) */
 
@@ -114,11 +114,12 @@ int tc_get_omega(tc_ctx* ctx, double* omega);
  * TC_PASSIVE class (default 0.05, :27). */
 int tc_set_smooth(tc_ctx* ctx, double smooth);
 int tc_get_smooth(tc_ctx* ctx, double* smooth);
-/* FP32C only: visit targets in the caller's order or along a Hilbert curve
- * over the six cube faces, continuous from face to face (default; results are
- * returned in the caller's order either way). The compensated arithmetic is
- * accurate when a CTA's targets are spatially close; the curve order
- * guarantees that for any input order. */
+/* Visit targets in the caller's order or along a Hilbert curve over the cube
+ * faces (default; results are returned in the caller's order either way). The
+ * compensated arithmetic is accurate when a CTA's targets are spatially close;
+ * the curve order guarantees that for any input order. FP64 is accurate in
+ * any order and faster with compact tiles: its targets are sorted in calls
+ * large enough for that to pay. */
 int tc_set_target_order(tc_ctx* ctx, int order);
 /* delta of each target class (reference: 0, 0, smooth). */
 int tc_set_deltas(tc_ctx* ctx, double delta_active, double delta_vertex, double delta_passive);
@@ -151,8 +152,8 @@ int tc_bs_velocity_device(tc_ctx* ctx, int target_class, const double* X, int m,
  * tc_bs_velocity_device's, capped by the space left. The scratch is a 32 MiB
  * array compiled into the library (held by every GPU that loads it): sources
  * 32*n bytes, partial sums 24*m per chunk and, for FP32C in the visiting
- * order, about 4*m + 20*(i1 - i0) for the order; a call for which one chunk
- * does not fit returns TC_ERR_ARG. The first call on a device (and the first
+ * order, about 4*m + 20*(i1 - i0) for the order (FP64 is sorted only where that
+ * fits too); a call for which one chunk does not fit returns TC_ERR_ARG. The first call on a device (and the first
  * after its context was re-created) looks the array's address up: make it
  * before any stream capture. Calls share the array, so calls that overlap on
  * the GPU race. */

@@ -146,7 +146,7 @@ int velocity_device(tc_ctx* ctx, int cls, const double* X, int m, const double* 
   if (rc) return rc;
   double4* src = ctx->scratch[0].as<double4>();
   int* perm = nullptr;
-  if (i1 > i0 && tcb::wants_order(ctx)) {
+  if (i1 > i0 && tcb::wants_order(ctx, i1 - i0, (double)(i1 - i0) * n)) {
     if ((rc = ctx->scratch[4].ensure((size_t)m * sizeof(int)))) return rc;
     perm = ctx->scratch[4].as<int>();
     const tcb::OrderJob job{X, i0, i1, perm, m, m};
@@ -585,9 +585,11 @@ extern "C" int tc_rk4_stage_range(tc_ctx* ctx, int stage, double dt, int a0, int
                          first ? R.x0V.as<double>() : R.xiV.as<double>(),
                          first ? R.x0Q.as<double>() : R.xiQ.as<double>()};
   const int range[6] = {a0, a1, v0, v1, q0, q1};
-  // FP32C visiting order: computed from the stage-0 positions once per step (targets move by
+  // visiting order: computed from the stage-0 positions once per step (targets move by
   // O(dt) within a step) and whenever the ranges change
-  const bool want_order = tcb::wants_order(ctx);
+  const long long most = std::max({a1 - a0, v1 - v0, q1 - q0});
+  const bool want_order =
+      tcb::wants_order(ctx, most, 4.0 * (double)R.nA * ((a1 - a0) + (v1 - v0) + (double)(q1 - q0)));
   if (!want_order) {
     R.ordered = false;
   } else if (first || !R.ordered || memcmp(range, R.order_range, sizeof(range)) != 0) {

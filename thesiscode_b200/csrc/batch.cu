@@ -180,7 +180,7 @@ int build_items(tc_ctx* ctx, tc_batch_plan& B, int variant, int chunk_len) {
 
 int upload_segments(tc_ctx* ctx, tc_batch_plan& B) {
   tcb::Rk4State& R = ctx->rk;
-  const bool ord = ctx->precision == TC_FP32C && R.ordered;
+  const bool ord = R.ordered;
   std::vector<tcb::BatchSeg> s0, s1;
   for (int b = 0; b < B.count; ++b)
     for (int cls = 0; cls < 2; ++cls) {
@@ -189,6 +189,7 @@ int upload_segments(tc_ctx* ctx, tc_batch_plan& B) {
       g.out_offset = cls == 0 ? 0 : B.nA_tot;
       g.self_offset = cls == 0 ? 0 : tcb::kNoSelf;
       g.d2 = ctx->delta[cls] * ctx->delta[cls];
+      g.compact = 1;
       g.perm_len = g.perm ? (long long)((cls == 0 ? R.permA : R.permV).bytes / sizeof(int)) : 0;
       g.x = cls == 0 ? R.x0A.as<double>() : R.x0V.as<double>();
       g.x_len = (long long)((cls == 0 ? R.x0A : R.x0V).bytes / (3 * sizeof(double)));
@@ -264,7 +265,7 @@ int enqueue_steps(tc_ctx* ctx, tc_batch_plan& B, double dt, int nsteps) {
 // default's accuracy (64-source FP32 flush; a 128-source flush is faster by
 // about 1% and raises the error by half).
 const int kTune32[] = {0, 1, 2, 3, 4, 5, 6, 7};
-const int kTune64[] = {2, 0, 1, 3};
+const int kTune64[] = {2, 0, 1, 3, 6, 7};
 
 // Times one stage-0 launch of the whole batch (best of `reps`).
 int time_launch(tc_ctx* ctx, tc_batch_plan& B, cudaEvent_t e0, cudaEvent_t e1, int reps,
@@ -381,7 +382,7 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
   TC_CUDA_TRY(cudaMemcpyAsync(B.cnt_d.ptr, cnt.data(), count * sizeof(int), cudaMemcpyHostToDevice,
                               ctx->stream));
   R.ordered = false;
-  if (ctx->precision == TC_FP32C && ctx->target_order == TC_ORDER_HILBERT) {
+  if (ctx->target_order == TC_ORDER_HILBERT) {
     int* ri = B.row_inst.as<int>();
     for (int cls = 0; cls < 2; ++cls) {
       const int n = cls == 0 ? B.nA_tot : B.nV_tot;

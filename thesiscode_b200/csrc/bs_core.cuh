@@ -24,11 +24,12 @@ constexpr int kNoSelf = INT32_MIN;
 
 struct TargetSeg {
   const double* x;  // targets, x[3*i + c]
-  const int* perm;  // FP32C: target at position p in [i0,i1) is perm[p] (null: p itself)
+  const int* perm;  // target at position p in [i0,i1) is perm[p] (null: p itself)
   int i0, i1;       // target range [i0, i1) computed by this launch
   int out_offset;   // partial row of target i is out_offset + i
   int self_offset;  // source index of target i is i + self_offset (ACTIVE), else kNoSelf
   double d2;        // delta^2 for this class
+  int compact;      // FP64: are tiles of these targets worth a look for a frame
   int tile_begin;   // first blockIdx.x of this segment
   long long x_len;     // checked build: points in x
   long long perm_len;  // checked build: entries in perm
@@ -56,22 +57,17 @@ struct UnitBounds {
 };
 
 // ---------------------------------------------------------------------------
-// Reciprocals. The hardware seed (rcp.approx) is refined by Newton-Raphson
-// r <- r + r(1 - d r); two steps take an FP64 seed to full precision. This
-// replaces the IEEE division of the reference (a ~14-DFMA sequence on this
-// GPU) by 4 DFMA; the result is within an ulp of 1/d.
+// Reciprocals. The hardware seed (rcp.approx.ftz.f64, relative error e0 below
+// 1e-6) takes one third-order step, r <- r (1 + e + e^2) with e = 1 - d r: the
+// error left is e0^3 < 1e-18, so 3 FMA give a result within an ulp of 1/d
+// (measured over [1, 2): 1.1e-16). Two Newton steps would take 4, the
+// compiler's IEEE division about 14.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double rcp_seed_f64(double d) {
+__device__ __forceinline__ double rcp_f64(double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  return r;
-}
-
-__device__ __forceinline__ double rcp_newton2(double d) {
-  double r = rcp_seed_f64(d);
   double e = fma(-d, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-d, r, 1.0);
+  e = fma(e, e, e);
   return fma(r, e, r);
 }
 
@@ -89,112 +85,360 @@ __device__ __forceinline__ const TargetSeg& find_seg(const PairLaunch& P, int ti
 }
 
 // ---------------------------------------------------------------------------
-// FP64 pair kernel.
+// Frames. A CTA with compact targets works in its own frame: an origin c on the
+// sphere near the middle of its targets and an orthonormal basis R = (e1, e2, e3)
+// with e3 along c. Points become offsets s = R (x - c).
 // ---------------------------------------------------------------------------
-// FUSED = false: the denominator is rounded exactly like the reference's
-// 1.0 - sum(...) (six separately rounded operations). FUSED = true: the
-// same expression as 1 - x.y + delta^2 in three fused multiply-adds, one
-// rounding instead of six; it differs from the reference's value by the
-// reference's own rounding error in the denominator (a few ulps of x.y).
-template <bool FUSED>
-__device__ __forceinline__ double pair_denominator(const double4& q, const double xi[3], double d2,
-                                                   double one_plus_d2) {
-  if (FUSED) {
-    double s = fma(-q.x, xi[0], one_plus_d2);
-    s = fma(-q.y, xi[1], s);
-    return fma(-q.z, xi[2], s);
+// Orthonormal basis with e3 = c/|c| (Duff, Burgess, Christensen, Hart, Kensler,
+// Liani, Pharr, "Building an Orthonormal Basis, Revisited", JCGT 6(1), 2017).
+__device__ __forceinline__ void make_frame(double cx, double cy, double cz, double* f) {
+  const double inv = rsqrt(fma(cx, cx, fma(cy, cy, cz * cz)));
+  const double nx = cx * inv, ny = cy * inv, nz = cz * inv;
+  const double sg = copysign(1.0, nz);
+  const double a = -1.0 / (sg + nz);
+  const double b = nx * ny * a;
+  f[0] = 1.0 + sg * nx * nx * a;
+  f[1] = sg * b;
+  f[2] = -sg * nx;
+  f[3] = b;
+  f[4] = sg + ny * ny * a;
+  f[5] = -ny;
+  f[6] = nx;
+  f[7] = ny;
+  f[8] = nz;
+}
+
+// R v with explicitly fused operations, so a target and the same point as a
+// source round identically.
+__device__ __forceinline__ double frame_dot(const double* e, double vx, double vy, double vz) {
+  return fma(e[0], vx, fma(e[1], vy, __dmul_rn(e[2], vz)));
+}
+
+// ---------------------------------------------------------------------------
+// FP64 pair kernel.
+//
+// The kernel is bound by the FP64 pipe, and there by the pair's operation
+// count and its register reads (a DFMA of three registers none of which the
+// instruction before it read takes 3.1 cycles a warp and scheduler, of two 2.1).
+// Two forms, chosen per CTA by how compact its targets are:
+//
+// * frame form (9 operations a pair), targets within kFrameRho of c: with
+//   x_k = c + s_k and x_i = c + t_i,
+//       1 + delta^2 - x_i.x_k = a_k (1 - b_i) + b_i' - s_k,1 t_i,1 - s_k,2 t_i,2,
+//       a_k = -c.s_k,  b_i = -c.t_i,  b_i' = b_i + delta^2 + (1 - |c|^2)
+//   holds for every x on or off the sphere (e3 is along c, so the third products
+//   of s.t are a_k b_i), and takes 3 FMA because the targets' part sits in
+//   registers. The sum is T' = sum_k r G_k R x_k: staging a source multiplies
+//   G_k in once per CTA, so a pair takes 3 FMA here, 3 there and 3 for the
+//   reciprocal. The multiple of x_i that T' carries (about sum r G, which
+//   u = x_i x T ignores) is taken out in the frame, where x_i is (small, small,
+//   about 1), before T' is rotated back. The denominator keeps an absolute error
+//   of ulps of |s| |t| where 1 - x.y keeps ulps of 1.
+// * wide form (13 operations), for targets all over the sphere: the fused
+//   1 - x.y + delta^2 of the global coordinates and sum_k w (x_k - x_i).
+//   STRICT variants always take it, with the denominator rounded like the
+//   reference's 1.0 - sum(...) + smooth*smooth (six separately rounded
+//   operations).
+//
+// Either way the sums of at most a tile's 256 sources are added to totals in shared
+// memory: in one long chain the sums' rounding would outweigh the terms'. Against
+// an extended-precision sum (levels 3-6, three fields, delta 0 and 0.01) the frame
+// form at |t| <= 0.7 has 0.1 to 1.0 times the error of the plain sum
+// sum_k w (x_k - x_i), and 1 to 2 times at |t| up to 2, hence the limit.
+//
+// Level 6 refined, 108,923 sources and 199,823 targets in three classes: 1.115e12
+// pairs/s with the wide form alone, at 14 operations, and now 1.53e12. 9 DFMA at
+// their nominal 2 cycles would allow 18.5e12 / 9 = 2.05e12; with the register reads
+// of a loop that shares a source among the targets (2.3 to 2.5 cycles) the bare loop
+// reaches 1.6e12.
+// ---------------------------------------------------------------------------
+constexpr float kFrameRho2 = 0.72f;  // frame form: |t|^2 at most (|t| <= 0.85)
+constexpr int kOwnTiles = 2048;     // bits of the own-tile map
+
+template <int NT, int TPT, int TS>
+struct Fp64Smem {
+  double2 a[TS];              // frame: (s_1, s_2); wide: (x, y)
+  double2 b[TS];              // frame: (a_k, G x'_1); wide: (z, G)
+  double2 c[TS];              // frame: (G x'_2, G x'_3)
+  double acc[3 * TPT * NT];   // totals [c][t][thread]
+  double frame[13];           // e1, e2, e3 (rows), c, 1 - |c|^2
+  double csum[4][NT / 32];    // per-warp sums of the target positions, and their number
+  unsigned own[kOwnTiles / 32];  // source tiles (mod kOwnTiles) that hold own points
+  unsigned rho[NT / 32];      // largest |t|^2, per warp
+  int framed;                 // a frame was found
+};
+
+// 1 - |c|^2 for |c| close to 1, without the rounding of |c|^2 to a double.
+__device__ __forceinline__ double one_minus_norm2(double cx, double cy, double cz) {
+  const double p[3] = {__dmul_rn(cx, cx), __dmul_rn(cy, cy), __dmul_rn(cz, cz)};
+  const double e[3] = {fma(cx, cx, -p[0]), fma(cy, cy, -p[1]), fma(cz, cz, -p[2])};
+  double hi = 1.0, lo = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {  // hi + lo = 1 - sum p (TwoSum)
+    const double s = __dsub_rn(hi, p[k]);
+    const double bb = __dsub_rn(s, hi);
+    lo = __dadd_rn(lo, __dadd_rn(__dsub_rn(hi, __dsub_rn(s, bb)), __dsub_rn(-p[k], bb)));
+    hi = s;
   }
-  double s = __dmul_rn(q.x, xi[0]);
-  s = __dadd_rn(s, __dmul_rn(q.y, xi[1]));
-  s = __dadd_rn(s, __dmul_rn(q.z, xi[2]));
+  return __dadd_rn(hi, __dsub_rn(lo, __dadd_rn(e[0], __dadd_rn(e[1], e[2]))));
+}
+
+// The wide form's denominator. STRICT: rounded exactly like the reference's
+// 1.0 - sum(...) + smooth*smooth.
+template <bool STRICT>
+__device__ __forceinline__ double wide_denominator(double qx, double qy, double qz, const double* xi,
+                                                   double d2, double one_plus_d2) {
+  if (!STRICT) return fma(-qz, xi[2], fma(-qy, xi[1], fma(-qx, xi[0], one_plus_d2)));
+  double s = __dmul_rn(qx, xi[0]);
+  s = __dadd_rn(s, __dmul_rn(qy, xi[1]));
+  s = __dadd_rn(s, __dmul_rn(qz, xi[2]));
   return __dadd_rn(__dsub_rn(1.0, s), d2);
 }
 
-// One work unit: the targets at positions [tile0, min(tile0 + NT*TPT, i_end))
-// of x against the sources [c0, c1); FP64 sums written to out[pos],
-// out[stride + pos], out[2*stride + pos]. Targets whose source index is
-// i + self_offset (self_offset != kNoSelf) skip themselves.
-template <int NT, int TPT, int TS, bool FUSED>
-__device__ __forceinline__ void fp64_unit(const double* __restrict__ x, int tile0, int i_end,
-                                          int self_offset, double d2,
-                                          const double4* __restrict__ src, int c0, int c1,
-                                          double* __restrict__ out, size_t stride, double4* sm,
-                                          const UnitBounds& ub) {
-  constexpr int TB = NT * TPT;
-  const double one_plus_d2 = 1.0 + d2;
-  const bool has_self = self_offset != kNoSelf;
-
-  double xi[TPT][3], acc[TPT][3];
-  int self_k[TPT];
+// Source j of the staged tile (index k) against the thread's targets. MASK: skip
+// the self pair, needed only in tiles that may hold the CTA's own points.
+template <int TPT, bool FRAME, bool STRICT, bool MASK, class Smem>
+__device__ __forceinline__ void fp64_source(const Smem& sm, int j, int k, const double (*tg)[4],
+                                            const int* self_k, double d2, double one_plus_d2,
+                                            double (*f)[3]) {
+  const double2 a = sm.a[j], b = sm.b[j];
+  double2 c = make_double2(0.0, 0.0);
+  if (FRAME) c = sm.c[j];
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {
-    int i = tile0 + (int)threadIdx.x + t * NT;
-    int ld = i < i_end ? i : tile0;
-    const bool okx = TC_BC(ub.rec, BC_PAIR_X, ld, ub.x_len);
-    xi[t][0] = okx ? x[3 * (size_t)ld] : 0.0;
-    xi[t][1] = okx ? x[3 * (size_t)ld + 1] : 0.0;
-    xi[t][2] = okx ? x[3 * (size_t)ld + 2] : 0.0;
-    acc[t][0] = acc[t][1] = acc[t][2] = 0.0;
-    self_k[t] = has_self ? i + self_offset : -1;
-  }
-  const int self_lo = has_self ? tile0 + self_offset : 0;
-  const int self_hi = has_self ? min(tile0 + TB, i_end) + self_offset : 0;
-
-  for (int ts = c0; ts < c1; ts += TS) {
-    __syncthreads();
-    for (int j = threadIdx.x; j < TS; j += NT) {
-      int k = ts + j;
-      sm[j] = (k < c1 && TC_BC(ub.rec, BC_PAIR_SRC, k, ub.src_len))
-                  ? src[k]
-                  : make_double4(0.0, 0.0, 0.0, 0.0);
-    }
-    __syncthreads();
-    const bool diag = has_self && ts < self_hi && self_lo < ts + TS;
-    if (!diag) {
-#pragma unroll 2
-      for (int j = 0; j < TS; ++j) {
-        const double4 q = sm[j];
-#pragma unroll
-        for (int t = 0; t < TPT; ++t) {
-          const double den = pair_denominator<FUSED>(q, xi[t], d2, one_plus_d2);
-          const double w = __dmul_rn(q.w, rcp_newton2(den));
-          acc[t][0] = fma(w, q.x - xi[t][0], acc[t][0]);
-          acc[t][1] = fma(w, q.y - xi[t][1], acc[t][1]);
-          acc[t][2] = fma(w, q.z - xi[t][2], acc[t][2]);
-        }
-      }
+    if (FRAME) {
+      double D = fma(b.x, tg[t][2], tg[t][3]);
+      D = fma(a.x, tg[t][0], D);
+      D = fma(a.y, tg[t][1], D);
+      double r = rcp_f64(D);
+      if (MASK) r = (k == self_k[t]) ? 0.0 : r;
+      f[t][0] = fma(r, b.y, f[t][0]);
+      f[t][1] = fma(r, c.x, f[t][1]);
+      f[t][2] = fma(r, c.y, f[t][2]);
     } else {
-      for (int j = 0; j < TS; ++j) {
-        const double4 q = sm[j];
-        const int k = ts + j;
-#pragma unroll
-        for (int t = 0; t < TPT; ++t) {
-          const double den = pair_denominator<FUSED>(q, xi[t], d2, one_plus_d2);
-          double w = __dmul_rn(q.w, rcp_newton2(den));
-          w = (k == self_k[t]) ? 0.0 : w;
-          acc[t][0] = fma(w, q.x - xi[t][0], acc[t][0]);
-          acc[t][1] = fma(w, q.y - xi[t][1], acc[t][1]);
-          acc[t][2] = fma(w, q.z - xi[t][2], acc[t][2]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < TPT; ++t) {
-    int i = tile0 + (int)threadIdx.x + t * NT;
-    if (i < i_end) {
-      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + i, ub.out_len)) out[i] = acc[t][0];
-      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + (long long)stride + i, ub.out_len))
-        out[stride + i] = acc[t][1];
-      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + 2 * (long long)stride + i, ub.out_len))
-        out[2 * stride + i] = acc[t][2];
+      const double D = wide_denominator<STRICT>(a.x, a.y, b.x, tg[t], d2, one_plus_d2);
+      double w = __dmul_rn(b.y, rcp_f64(D));
+      if (MASK) w = (k == self_k[t]) ? 0.0 : w;
+      f[t][0] = fma(w, a.x - tg[t][0], f[t][0]);
+      f[t][1] = fma(w, a.y - tg[t][1], f[t][1]);
+      f[t][2] = fma(w, b.x - tg[t][2], f[t][2]);
     }
   }
 }
 
-template <int NT, int TPT, int TS, int MINB, bool FUSED>
+// Sources [c0, c1) against the thread's targets, totals in sm.acc. SHORT: the last
+// tile is staged and walked to its end only (a chunk need not be whole tiles);
+// otherwise it is padded, and the loop's length is known when it is compiled.
+template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool FRAME, bool STRICT, class Smem>
+__device__ __forceinline__ void fp64_sum(const double4* __restrict__ src, int c0, int c1, Smem& sm,
+                                         const double (*tg)[4], const int* self_k, bool idle,
+                                         double d2, const UnitBounds& ub) {
+  const double one_plus_d2 = 1.0 + d2;
+  double f[TPT][3];
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) f[t][0] = f[t][1] = f[t][2] = 0.0;
+  for (int ts = c0; ts < c1; ts += TS) {
+    __syncthreads();
+    const int len = SHORT ? min(TS, (c1 - ts + UNROLL - 1) / UNROLL * UNROLL) : TS;
+    for (int j = threadIdx.x; j < len; j += NT) {
+      const int k = ts + j;
+      // padding: zero weight and (frame) a denominator of at least 1 off the targets
+      double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
+      const bool in = k < c1 && TC_BC(ub.rec, BC_PAIR_SRC, k, ub.src_len);
+      if (in) q = src[k];
+      if (FRAME) {
+        const double* fr = sm.frame;
+        const double dx = q.x - fr[9], dy = q.y - fr[10], dz = q.z - fr[11];
+        const double s1 = frame_dot(fr, dx, dy, dz), s2 = frame_dot(fr + 3, dx, dy, dz),
+                     ak = -frame_dot(fr + 9, dx, dy, dz);
+        sm.a[j] = in ? make_double2(s1, s2) : make_double2(0.0, 0.0);
+        sm.b[j] = in ? make_double2(ak, __dmul_rn(q.w, s1)) : make_double2(1.0, 0.0);
+        sm.c[j] = in ? make_double2(__dmul_rn(q.w, s2), fma(-q.w, ak, q.w)) : make_double2(0.0, 0.0);
+      } else {
+        sm.a[j] = make_double2(q.x, q.y);
+        sm.b[j] = make_double2(q.z, q.w);
+      }
+    }
+    __syncthreads();
+    if (idle) continue;  // a warp past the last target only stages
+    const int tile = (ts - c0) / TS % kOwnTiles;
+    if ((sm.own[tile / 32] >> (tile % 32)) & 1u) {
+#pragma unroll UNROLL
+      for (int j = 0; j < len; ++j)
+        fp64_source<TPT, FRAME, STRICT, true>(sm, j, ts + j, tg, self_k, d2, one_plus_d2, f);
+    } else {
+#pragma unroll UNROLL
+      for (int j = 0; j < len; ++j)
+        fp64_source<TPT, FRAME, STRICT, false>(sm, j, ts + j, tg, self_k, d2, one_plus_d2, f);
+    }
+#pragma unroll
+    for (int t = 0; t < TPT; ++t)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sm.acc[(c * TPT + t) * NT + threadIdx.x] += f[t][c];
+        f[t][c] = 0.0;
+      }
+  }
+}
+
+// One work unit: the targets at visiting positions [tile0, min(tile0 + NT*TPT,
+// i_end)) against the sources [c0, c1); FP64 sums written to out[pos],
+// out[stride + pos], out[2*stride + pos]. A target whose index is i has the
+// source index i + self_offset and skips itself (self_offset != kNoSelf).
+template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool STRICT>
+__device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const int* __restrict__ perm,
+                                          int tile0, int i_end, int self_offset, double d2,
+                                          bool compact, const double4* __restrict__ src, int c0,
+                                          int c1, double* __restrict__ out, size_t stride,
+                                          Fp64Smem<NT, TPT, TS>& sm, const UnitBounds& ub) {
+  static_assert(TS == 256 && TS % UNROLL == 0, "256 sources between additions to the totals");
+  const bool has_self = self_offset != kNoSelf;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+
+  double xi[TPT][3];
+  int self_k[TPT];
+  double px = 0.0, py = 0.0, pz = 0.0, pn = 0.0;
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) {
+    const int pos = tile0 + (int)threadIdx.x + t * NT;
+    const bool valid = pos < i_end;
+    const int p = valid ? pos : tile0;
+    int ld = p;
+    if (perm) ld = TC_BC(ub.rec, BC_PAIR_PERM, p, ub.perm_len) ? perm[p] : 0;
+    const bool okx = TC_BC(ub.rec, BC_PAIR_X, ld, ub.x_len);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) xi[t][c] = okx ? x[3 * (size_t)ld + c] : 0.0;
+    self_k[t] = has_self && valid ? ld + self_offset : -1;
+    // points far off the sphere (or not finite) have no say in the origin
+    const double n2 = fma(xi[t][0], xi[t][0], fma(xi[t][1], xi[t][1], xi[t][2] * xi[t][2]));
+    if (!STRICT && compact && valid && n2 > 0.25 && n2 < 4.0) {
+      px += xi[t][0];
+      py += xi[t][1];
+      pz += xi[t][2];
+      pn += 1.0;
+    }
+  }
+  if (!STRICT && compact) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      px += __shfl_xor_sync(0xffffffffu, px, o);
+      py += __shfl_xor_sync(0xffffffffu, py, o);
+      pz += __shfl_xor_sync(0xffffffffu, pz, o);
+      pn += __shfl_xor_sync(0xffffffffu, pn, o);
+    }
+  }
+  __syncthreads();  // the previous unit (persistent kernel) is done with the shared memory
+  if (!STRICT && lane == 0) {
+    sm.csum[0][warp] = px;
+    sm.csum[1][warp] = py;
+    sm.csum[2][warp] = pz;
+    sm.csum[3][warp] = pn;
+  }
+  for (int k = threadIdx.x; k < kOwnTiles / 32; k += NT) sm.own[k] = 0u;
+#pragma unroll
+  for (int k = 0; k < 3 * TPT; ++k) sm.acc[k * NT + threadIdx.x] = 0.0;
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < TPT; ++t)
+    if (self_k[t] >= c0 && self_k[t] < c1) {
+      const int tile = (self_k[t] - c0) / TS % kOwnTiles;
+      atomicOr(&sm.own[tile / 32], 1u << (tile % 32));
+    }
+  bool frame = false;
+  double tg[TPT][4];  // frame: -t_1, -t_2, 1 - b_i, b_i'; wide: x, y, z
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) {
+    tg[t][0] = xi[t][0];
+    tg[t][1] = xi[t][1];
+    tg[t][2] = xi[t][2];
+    tg[t][3] = 0.0;
+  }
+  if (!STRICT && compact) {
+    if (threadIdx.x == 0) {
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, n = 0.0;
+      for (int w = 0; w < NT / 32; ++w) {
+        s0 += sm.csum[0][w];
+        s1 += sm.csum[1][w];
+        s2 += sm.csum[2][w];
+        n += sm.csum[3][w];
+      }
+      const double n2 = fma(s0, s0, fma(s1, s1, s2 * s2));
+      sm.framed = n2 > 0.25 * n * n;  // else the targets surround the centre
+      if (sm.framed) {
+        const double inv = rsqrt(n2);
+        const double cx = s0 * inv, cy = s1 * inv, cz = s2 * inv;
+        make_frame(cx, cy, cz, sm.frame);
+        sm.frame[9] = cx;
+        sm.frame[10] = cy;
+        sm.frame[11] = cz;
+        sm.frame[12] = one_minus_norm2(cx, cy, cz);
+      }
+    }
+    __syncthreads();
+    if (sm.framed) {
+      const double* fr = sm.frame;
+      float rho2 = 0.f;
+#pragma unroll
+      for (int t = 0; t < TPT; ++t) {
+        const double dx = xi[t][0] - fr[9], dy = xi[t][1] - fr[10], dz = xi[t][2] - fr[11];
+        const double t1 = frame_dot(fr, dx, dy, dz), t2 = frame_dot(fr + 3, dx, dy, dz),
+                     bi = -frame_dot(fr + 9, dx, dy, dz);
+        rho2 = fmaxf(rho2, (float)fma(dx, dx, fma(dy, dy, dz * dz)));
+        tg[t][0] = -t1;
+        tg[t][1] = -t2;
+        tg[t][2] = 1.0 - bi;
+        tg[t][3] = bi + (d2 + fr[12]);
+      }
+      const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(rho2));
+      if (lane == 0) sm.rho[warp] = m;
+      __syncthreads();
+      unsigned r = 0;
+#pragma unroll
+      for (int w = 0; w < NT / 32; ++w) r = max(r, sm.rho[w]);
+      frame = __uint_as_float(r) <= kFrameRho2;
+      if (!frame) {
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+          tg[t][0] = xi[t][0];
+          tg[t][1] = xi[t][1];
+          tg[t][2] = xi[t][2];
+        }
+      }
+    }
+  }
+  const bool idle = tile0 + warp * 32 >= i_end;
+  if (frame)
+    fp64_sum<NT, TPT, TS, UNROLL, SHORT, true, false>(src, c0, c1, sm, tg, self_k, idle, d2, ub);
+  else
+    fp64_sum<NT, TPT, TS, 2, SHORT, false, STRICT>(src, c0, c1, sm, tg, self_k, idle, d2, ub);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) {
+    const int i = tile0 + (int)threadIdx.x + t * NT;
+    double T[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) T[c] = sm.acc[(c * TPT + t) * NT + threadIdx.x];
+    if (frame) {
+      // out with the multiple of x'_i = (t_1, t_2, 1 - b_i), then back: T = R^T T'
+      const double* fr = sm.frame;
+      const double v0 = -tg[t][0], v1 = -tg[t][1], v2 = tg[t][2];
+      const double lam = fma(T[0], v0, fma(T[1], v1, T[2] * v2)) / fma(v0, v0, fma(v1, v1, v2 * v2));
+      const double a0 = fma(-lam, v0, T[0]), a1 = fma(-lam, v1, T[1]), a2 = fma(-lam, v2, T[2]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) T[c] = fma(fr[c], a0, fma(fr[3 + c], a1, fr[6 + c] * a2));
+    }
+    if (i < i_end) {
+      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + i, ub.out_len)) out[i] = T[0];
+      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + (long long)stride + i, ub.out_len))
+        out[stride + i] = T[1];
+      if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + 2 * (long long)stride + i, ub.out_len))
+        out[2 * stride + i] = T[2];
+    }
+  }
+}
+
+template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P) {
-  __shared__ double4 sm[TS];
+  __shared__ Fp64Smem<NT, TPT, TS> sm;
   const TargetSeg& G = find_seg(P, blockIdx.x);
   const int tile0 = G.i0 + (int)(blockIdx.x - G.tile_begin) * (NT * TPT);
   const int c0 = (int)blockIdx.y * P.chunk_len;
@@ -203,8 +447,9 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P)
   const long long base = (long long)blockIdx.y * 3 * (long long)stride + G.out_offset;
   double* out = P.partial + base;
   const UnitBounds ub{P.bc, G.x_len, G.perm_len, P.src_len, base, P.partial_len};
-  fp64_unit<NT, TPT, TS, FUSED>(G.x, tile0, G.i1, G.self_offset, G.d2, P.src, c0, c1, out, stride,
-                                sm, ub);
+  fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT>(
+      G.x, G.perm, tile0, G.i1, G.self_offset, G.d2, G.compact != 0, P.src, c0, c1, out, stride, sm,
+      ub);
 }
 
 // ---------------------------------------------------------------------------
@@ -323,31 +568,6 @@ struct SpSmem {
   unsigned tmin[NT / 32];
   unsigned rho[NT / 32];
 };
-
-// Orthonormal basis with e3 = c/|c| (Duff, Burgess, Christensen, Hart, Kensler,
-// Liani, Pharr, "Building an Orthonormal Basis, Revisited", JCGT 6(1), 2017).
-__device__ __forceinline__ void make_frame(double cx, double cy, double cz, double* f) {
-  const double inv = rsqrt(fma(cx, cx, fma(cy, cy, cz * cz)));
-  const double nx = cx * inv, ny = cy * inv, nz = cz * inv;
-  const double sg = copysign(1.0, nz);
-  const double a = -1.0 / (sg + nz);
-  const double b = nx * ny * a;
-  f[0] = 1.0 + sg * nx * nx * a;
-  f[1] = sg * b;
-  f[2] = -sg * nx;
-  f[3] = b;
-  f[4] = sg + ny * ny * a;
-  f[5] = -ny;
-  f[6] = nx;
-  f[7] = ny;
-  f[8] = nz;
-}
-
-// R v with explicitly fused operations, so a target and the same point as a
-// source round identically (the self pair then has d = 0 exactly).
-__device__ __forceinline__ double frame_dot(const double* e, double vx, double vy, double vz) {
-  return fma(e[0], vx, fma(e[1], vy, __dmul_rn(e[2], vz)));
-}
 
 __device__ __forceinline__ float2 rcp2(float2 D) {
   return make_float2(rcp_approx_f32(D.x), rcp_approx_f32(D.y));
@@ -728,10 +948,11 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp32c_kernel(const PairLaunch P
 // ---------------------------------------------------------------------------
 struct BatchSeg {
   const double* x;   // target positions of the class (concatenated instances)
-  const int* perm;   // FP32C visiting order (null: as stored)
+  const int* perm;   // visiting order (null: as stored)
   int out_offset;    // partial row of target position p is out_offset + p
   int self_offset;   // TC_ACTIVE: source index of target i is i + self_offset
   double d2;
+  int compact;       // FP64: are tiles of these targets worth a look for a frame
   long long x_len;     // checked build: points in x
   long long perm_len;  // checked build: entries in perm
 };
@@ -781,9 +1002,9 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp32c_batch_kernel(const BatchL
   }
 }
 
-template <int NT, int TPT, int TS, int MINB, bool FUSED>
+template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_batch_kernel(const BatchLaunch B) {
-  __shared__ double4 sm[TS];
+  __shared__ Fp64Smem<NT, TPT, TS> sm;
   __shared__ int slot;
   for (int it = next_item(B.counter, &slot); it < B.n_items; it = next_item(B.counter, &slot)) {
     const BatchItem I = B.items[it];
@@ -792,8 +1013,9 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_batch_kernel(const BatchLa
     const long long base = (long long)I.chunk * 3 * (long long)B.stride + S.out_offset;
     double* out = B.partial + base;
     const UnitBounds ub{B.bc, S.x_len, S.perm_len, B.src_len, base, B.partial_len};
-    fp64_unit<NT, TPT, TS, FUSED>(S.x, I.tile0, I.i1, S.self_offset, S.d2, B.src, I.c0, I.c1, out,
-                                  B.stride, sm, ub);
+    fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT>(
+        S.x, S.perm, I.tile0, I.i1, S.self_offset, S.d2, S.compact != 0, B.src, I.c0, I.c1, out,
+        B.stride, sm, ub);
   }
 }
 

@@ -41,13 +41,13 @@ void DevBuf::release() {
 // ---------------------------------------------------------------------------
 constexpr int kTS = 256;
 
-template <int NT, int TPT, int MINB, bool FUSED, int TS>
+template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64(dim3 g, cudaStream_t s, const PairLaunch& P) {
-  pair_fp64_kernel<NT, TPT, TS, MINB, FUSED><<<g, NT, 0, s>>>(P);
+  pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT><<<g, NT, 0, s>>>(P);
 }
-template <int NT, int TPT, int MINB, bool FUSED, int TS>
+template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64b(int g, cudaStream_t s, const BatchLaunch& B) {
-  pair_fp64_batch_kernel<NT, TPT, TS, MINB, FUSED><<<g, NT, 0, s>>>(B);
+  pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT><<<g, NT, 0, s>>>(B);
 }
 template <int NT, int T, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32b(int g, cudaStream_t s, const BatchLaunch& B) {
@@ -58,12 +58,12 @@ void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
   pair_fp32c_kernel<NT, T, kTS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(P);
 }
 
-#define V64T(NT, TPT, MINB, FUSED, TS)                                              \
-  PairVariant { TC_FP64, NT, TPT, TS, FUSED, MINB, 0, launch64<NT, TPT, MINB, FUSED, TS>, \
-                (const void*)pair_fp64_kernel<NT, TPT, TS, MINB, FUSED>,                  \
-                launch64b<NT, TPT, MINB, FUSED, TS>,                                        \
-                (const void*)pair_fp64_batch_kernel<NT, TPT, TS, MINB, FUSED>, 0 }
-#define V64(NT, TPT, MINB, FUSED) V64T(NT, TPT, MINB, FUSED, kTS)
+#define V64(NT, TPT, MINB, UNROLL, SHORT, STRICT)                                            \
+  PairVariant { TC_FP64, NT, TPT, kTS, !STRICT, MINB, UNROLL,                                 \
+                launch64<NT, TPT, MINB, UNROLL, SHORT, STRICT>,                               \
+                (const void*)pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>,     \
+                launch64b<NT, TPT, MINB, UNROLL, SHORT, STRICT>,                              \
+                (const void*)pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, 0 }
 // FP32C: T targets per thread, FP32 flush every FLUSH sources, form bits FM
 #define V32(NT, T, FLUSH, MINB, UNROLL, FM)                                            \
   PairVariant { TC_FP32C, NT, T, kTS, FLUSH, MINB, UNROLL,                             \
@@ -74,13 +74,19 @@ void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
 
 // FP64: the `flush` field records the denominator mode (1 = fused, 0 =
 // rounded exactly like the reference).
-// Variant 6 is variant 2 with 32-source tiles, for launches too small to fill
-// one wave of whole 256-source chunks (chosen automatically, fp64_small).
+// 2: default. 6 and 7: launches over few sources or targets, chosen automatically
+// (auto64_variant); 4 and 5: the reference's rounding; 0, 1 and 3: shapes the batch
+// autotuner may choose. Six targets a thread share each source's registers and leave
+// 8 warps an SM, which the six independent pairs feed (level 6, 1e10 pairs, ms a
+// launch: 2 targets 6.87, 3 6.77, 4 6.62, 5 6.53, 6 6.41, 8 6.60).
 const PairVariant kVariants64[] = {
-    V64(256, 2, 5, true),  V64(256, 4, 2, true),  V64(256, 1, 6, true), V64(128, 4, 4, true),
-    V64(256, 2, 5, false), V64(256, 4, 2, false), V64T(256, 1, 6, true, 32),
+    V64(128, 5, 3, 2, false, false), V64(256, 4, 2, 2, false, false),
+    V64(128, 6, 2, 4, false, false), V64(64, 6, 4, 2, false, false),
+    V64(256, 2, 4, 2, false, true),  V64(256, 4, 2, 2, false, true),
+    V64(32, 4, 12, 2, true, false),  V64(64, 6, 4, 2, true, false),
 };
-static_assert(kAuto64Default == 2 && kAuto64Small == 6, "automatic FP64 variants");
+static_assert(kAuto64Default == 2 && kAuto64Small == 6 && kAuto64Mid == 7,
+              "automatic FP64 variants");
 // FP32C form bits (SpForm in bs_core.cuh): 8 = source-paired form (all
 // variants), 2 = FP64 accumulators in shared memory, 4 = hi/lo near offsets,
 // 256 / 512 = tiles whose every source is far flushed every 2 / 4 flush
@@ -178,25 +184,29 @@ static int choose_chunks(int tiles, int n, int ts, int slots, int min_chunk, int
   return best;
 }
 
-// Source chunk length of an FP64 launch too small to fill the GPU with
-// whole 256-source chunks (run with kAuto64Small's 32-source tiles, so that
-// chunks may be any multiple of 32 sources without padding). The work items run
-// in one or two waves, and each SM works through its CTAs at its FP64 pipe's
-// rate. The length minimised is therefore ceil(items / SMs) x chunk length.
-// Example: 5,120 sources and 31 tiles on 148 SMs. Whole-tile chunks allow at
-// most 20 chunks: 620 items, 5 per SM, of 256 sources each (1,280). Chunks of
-// 224 give 23 chunks: 713 items, 5 per SM, 1,120 (-12.5%).
-static int fine_chunk_len(int tiles, int n, int num_sms, int slots, int max_chunks, int gran) {
-  long long best_cost = -1;
+constexpr int kFullWarps = 12;
+constexpr int kRoundSources = 64;
+
+// Source chunk length of an FP64 launch, by a model of its time. The CTAs of one
+// chunk walk len sources each; an SM holds `resident` of them at a time and needs
+// kFullWarps warps for the FP64 pipe's full rate, so a round of c CTAs takes len x
+// max(c, enough) (enough CTAs for that many warps) and, for its prologue, epilogue
+// and staging, about as long as kRoundSources more. Chunks are multiples of gran.
+static int fine_chunk_len(int tiles, int n, int num_sms, int slots, int warps, int max_chunks,
+                          int gran) {
+  const int resident = std::max(1, slots / num_sms);
+  const int enough = std::max(1, std::min(resident, kFullWarps / warps));
+  double best_cost = -1.0;
   int best_len = n;
   for (int s = 1; s <= max_chunks; ++s) {
     int len = (n + s - 1) / s;
     len = (len + gran - 1) / gran * gran;
     const int chunks = (n + len - 1) / len;
-    const long long items = (long long)tiles * chunks;
-    if (items > 2LL * slots) break;
-    const long long cost = (items + num_sms - 1) / num_sms * (long long)len;
-    if (best_cost < 0 || cost < best_cost) {
+    const long long per_sm = ((long long)tiles * chunks + num_sms - 1) / num_sms;
+    const long long full = per_sm / resident, rest = per_sm % resident;
+    const double load = (double)full * resident + (rest ? std::max<long long>(rest, enough) : 0);
+    const double cost = load * len + (double)kRoundSources * enough * (double)(full + (rest ? 1 : 0));
+    if (best_cost < 0.0 || cost < best_cost * 0.995) {
       best_cost = cost;
       best_len = len;
     }
@@ -211,14 +221,34 @@ static int whole_chunk_len(int tiles, int n, int ts, int slots, int min_chunk, i
   return (len + ts - 1) / ts * ts;
 }
 
-// With the default FP64 variant's whole-tile chunks, does this launch fill
-// less than 90% of one wave's CTA slots?
-static bool fp64_small(const tc_ctx* ctx, int tiles, int n, int max_chunks) {
+static int count_tiles(const SegDesc* segs, int nseg, int tb) {
+  int tiles = 0;
+  for (int s = 0; s < nseg; ++s) tiles += std::max(0, segs[s].i1 - segs[s].i0 + tb - 1) / tb;
+  return tiles;
+}
+
+// Automatic FP64 variant. The default's tiles of 768 targets leave SMs idle when
+// its whole-tile chunks fill less than 90% of one wave, and on coarse grids they
+// reach past the frame form's limit and cut the work into too few pieces: below
+// 12,288 sources tiles of 128 targets are faster (pair launch at levels 3 / 4 / 4
+// refined to 6,023: 12.6 / 43 / 55 us, tiles of 384: 11.2 / 49 / 63), below 65,536
+// tiles of 384 (level 5: 0.454 ms, of 128 0.496, of 768 0.49), from there on 768
+// (level 6: 6.41 ms, of 384 6.54).
+constexpr int kFewSources = 12288, kMidSources = 65536;
+
+static int auto64_variant(const tc_ctx* ctx, const SegDesc* segs, int nseg, int n, int max_chunks) {
+  const PairVariant& v = kVariants64[kAuto64Default];
+  const int tiles = count_tiles(segs, nseg, v.nt * v.tpt);
   const int slots = ctx->slots64_default;
   const int len = whole_chunk_len(tiles, n, kTS, slots, ctx->min_chunk, max_chunks);
   const long long items = (long long)tiles * ((n + len - 1) / len);
-  return items * 10 < 9LL * slots;
+  if (items * 10 < 9LL * slots || n < kFewSources) return kAuto64Small;
+  return n < kMidSources ? kAuto64Mid : kAuto64Default;
 }
+
+// A tile of 1/8 of the sphere's targets has a radius of about 0.7 at best, the
+// frame form's limit: fewer tiles than that are not worth the search for a frame.
+constexpr int kCompactTiles = 8;
 
 // Tiles and chunking of one pair launch: the target segments, the grid and the
 // chunk length (partial sums need S * 3 * n_out doubles).
@@ -229,8 +259,15 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
     const int rc0 = use_fp32c_variant(ctx, n);
     if (rc0) return rc0;
   }
-  const PairCfg& cfg = fp64 ? ctx->cfg64 : ctx->cfg32;
-  const int tb = cfg.tb();
+  if (fp64 && ctx->auto64 && n > 0 && count_tiles(segs, nseg, 1) > 0) {
+    const int want = auto64_variant(ctx, segs, nseg, n, max_chunks);
+    if (want != ctx->var64) {
+      const int rc = select_variant(ctx, TC_FP64, want);
+      if (rc) return rc;
+    }
+  }
+  const PairCfg& cur = fp64 ? ctx->cfg64 : ctx->cfg32;
+  const int tb = cur.tb();
   *P = PairLaunch{};
   int tiles = 0, k = 0;
   for (int s = 0; s < nseg; ++s) {
@@ -238,12 +275,13 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
     if (len <= 0) continue;
     TargetSeg& g = P->seg[k++];
     g.x = segs[s].x;
-    g.perm = fp64 ? nullptr : segs[s].perm;
+    g.perm = segs[s].perm;
     g.i0 = segs[s].i0;
     g.i1 = segs[s].i1;
     g.out_offset = segs[s].out_offset;
     g.self_offset = segs[s].self_offset;
     g.d2 = segs[s].d2;
+    g.compact = len >= kCompactTiles * tb;
     g.x_len = bc_extent(ctx, BC_PAIR_X, segs[s].x_len);
     g.perm_len = bc_extent(ctx, BC_PAIR_PERM, segs[s].perm_len);
     g.tile_begin = tiles;
@@ -252,19 +290,11 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
   P->nseg = k;
   *grid = dim3(tiles, 0);
   if (tiles == 0 || n <= 0) return TC_OK;
-  // automatic FP64 variant: the same target tiles either way, only the source tiles differ
-  if (fp64 && ctx->auto64) {
-    const int want = fp64_small(ctx, tiles, n, max_chunks) ? kAuto64Small : kAuto64Default;
-    if (want != ctx->var64) {
-      const int rc = select_variant(ctx, TC_FP64, want);
-      if (rc) return rc;
-    }
-  }
-  const PairCfg& cur = fp64 ? ctx->cfg64 : ctx->cfg32;
   const int slots = fp64 ? ctx->slots64 : ctx->slots32;
   const int chunk_len =
-      (fp64 && ctx->auto64 && ctx->var64 == kAuto64Small)
-          ? fine_chunk_len(tiles, n, ctx->num_sms, slots, max_chunks, cur.ts)
+      (fp64 && ctx->auto64)
+          ? fine_chunk_len(tiles, n, ctx->num_sms, slots, cur.nt / 32, max_chunks,
+                           ctx->var64 == kAuto64Default ? cur.ts : 16)
           : whole_chunk_len(tiles, n, cur.ts, slots, ctx->min_chunk, max_chunks);
   const int S = (n + chunk_len - 1) / chunk_len;
   P->src = src;
@@ -499,7 +529,6 @@ int launch_velocity_epilogue(tc_ctx* ctx, const double* x, const int* perm, int 
     partial = ctx->partial.as<double>();
     partial_len = (long long)(ctx->partial.bytes / sizeof(double));
   }
-  if (ctx->precision == TC_FP64) perm = nullptr;
   const EpiBounds eb{ctx->bc_rec, bc_extent(ctx, BC_EPI_X, m), bc_extent(ctx, BC_EPI_PERM, m),
                      bc_extent(ctx, BC_EPI_PARTIAL, partial_len), bc_extent(ctx, BC_EPI_OUT, m)};
   velocity_epilogue_kernel<<<(m + 255) / 256, 256, 0, ctx->stream>>>(
@@ -706,7 +735,7 @@ int launch_stage_epilogue(tc_ctx* ctx, int stage, double dt, const int range[6],
   E.src = R.src.as<double4>();
   E.ke = R.ke.as<double>();
   E.keBlocks = R.keBlocks.as<double>();
-  const bool ordered = ctx->precision != TC_FP64 && R.ordered;
+  const bool ordered = R.ordered;
   E.permA = ordered ? R.permA.as<int>() : nullptr;
   E.permV = ordered ? R.permV.as<int>() : nullptr;
   E.permQ = ordered ? R.permQ.as<int>() : nullptr;

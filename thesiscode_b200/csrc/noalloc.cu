@@ -16,7 +16,9 @@
 // exits. A call needs 32*n bytes for the sources (each part rounded up to 256
 // bytes), 24*m per source chunk for the partial sums and, for FP32C with the
 // library's visiting order, 4*m for the order plus about 20 bytes per target
-// in range [i0, i1) for its sort; larger calls are rejected with TC_ERR_ARG.
+// in range [i0, i1) for its sort; larger calls are rejected with TC_ERR_ARG. FP64
+// calls that the allocating entry point would sort are sorted if that fits, and run
+// in the stored order if not.
 // The chunk count is the allocating entry point's choice, capped by what fits,
 // so the two entry points give the same result whenever that choice fits.
 //
@@ -146,15 +148,23 @@ extern "C" int tc_bs_velocity_device_noalloc(tc_ctx* ctx, int target_class, cons
   }
   // layout: sources | order (perm, keys in, keys out, indices, sort temp) | partial sums
   const int len = i1 - i0;
-  const bool ordered = ctx->precision == TC_FP32C && ctx->target_order == TC_ORDER_HILBERT && len > 0;
+  bool ordered = len > 0 && tcb::wants_order(ctx, len, (double)len * n);
   size_t sort_bytes = 0;
   int rc;
   if (ordered && (rc = tcb::order_sort_bytes(len, &sort_bytes))) return rc;
   const size_t src_bytes = round256((size_t)n * sizeof(double4));
-  const size_t perm_bytes = ordered ? round256((size_t)m * sizeof(int)) : 0;
-  const size_t key_bytes = ordered ? round256((size_t)len * sizeof(unsigned)) : 0;
-  const size_t order_bytes = ordered ? perm_bytes + 3 * key_bytes + round256(sort_bytes) : 0;
   const size_t chunk_bytes = 3 * (size_t)m * sizeof(double);
+  size_t perm_bytes = 0, key_bytes = 0, order_bytes = 0;
+  if (ordered) {
+    perm_bytes = round256((size_t)m * sizeof(int));
+    key_bytes = round256((size_t)len * sizeof(unsigned));
+    order_bytes = perm_bytes + 3 * key_bytes + round256(sort_bytes);
+    // FP64 targets are sorted for speed only: without room for that they are visited as stored
+    if (ctx->precision == TC_FP64 && src_bytes + order_bytes + chunk_bytes > kNoAllocScratchBytes) {
+      ordered = false;
+      perm_bytes = key_bytes = order_bytes = 0;
+    }
+  }
   const size_t fixed = src_bytes + order_bytes;
   if (fixed > kNoAllocScratchBytes || (len > 0 && n > 0 && kNoAllocScratchBytes - fixed < chunk_bytes)) {
     tc_record_error("tc_bs_velocity_device_noalloc: n=%d sources and m=%d targets need %zu bytes of "

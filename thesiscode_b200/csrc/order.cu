@@ -1,5 +1,4 @@
-// Spatially coherent visiting order of targets for the FP32-compensated pair
-// kernel: each target is keyed by its cube face and its position along a 2-D
+// Spatially coherent visiting order of targets for the pair kernels: each target is keyed by its cube face and its position along a 2-D
 // Hilbert curve over that face (sphere_order.cuh) and the keys are sorted with
 // a stable radix sort, so a CTA's consecutive targets form a compact patch of
 // the sphere whatever order the caller stores them in (the reference numbers
@@ -252,9 +251,18 @@ int compute_orders(tc_ctx* ctx, const OrderJob* jobs, int count) {
   return TC_OK;
 }
 
-// Are targets visited in that order? (FP32C: its near form wants compact tiles.)
-bool wants_order(const tc_ctx* ctx) {
-  return ctx->precision == TC_FP32C && ctx->target_order == TC_ORDER_HILBERT;
+// FP64 targets are visited in order where that pays. The refinement's panel order
+// is compact already, the particles' creation order is not, and a CTA whose targets
+// lie all over the sphere runs the 13-operation wide form instead of the 9-operation
+// frame form. Pair launches in the given order and sorted: level 4 (3.9e7 pairs)
+// 45.5 and 43.3 us, level 4 refined (6.7e7) 61.7 and 54.5, level 5 (6.3e8) 515 and
+// 455; the sort's two launches take 13 to 18 us once in a step of four. So: from
+// 2e8 pairs a call, and 2,048 targets, below which a tile covers too much of the
+// sphere for the frame form.
+bool wants_order(const tc_ctx* ctx, long long most_targets, double pairs) {
+  if (ctx->target_order != TC_ORDER_HILBERT) return false;
+  if (ctx->precision == TC_FP32C) return true;
+  return most_targets >= 2048 && pairs >= 2e8;
 }
 
 }  // namespace tcb

@@ -48,7 +48,7 @@ struct PairVariant {
 // Target segment as the host describes it before tiles are assigned.
 struct SegDesc {
   const double* x;
-  const int* perm;  // visiting order of [i0, i1) (FP32C only; null: as stored)
+  const int* perm;  // visiting order of [i0, i1) (null: as stored)
   int i0, i1;
   int out_offset;
   int self_offset;
@@ -70,7 +70,7 @@ struct Rk4State {
   DevBuf ke;                            // kineticEnergy(nA), stage 1
   DevBuf keBlocks;                      // per-block partial sums of KE*A
   DevBuf totalKE;                       // one value per step
-  DevBuf permA, permV, permQ;           // FP32C visiting orders (cube-face Hilbert), per class
+  DevBuf permA, permV, permQ;           // visiting orders (cube-face Hilbert), per class
   bool ordered = false;                 // perm* hold orders of the current stage ranges
   int order_range[6] = {0, 0, 0, 0, 0, 0};
   // forced (stratosphere) model: source vorticity rebuilt each stage from absA
@@ -97,13 +97,13 @@ struct tc_ctx {
   int num_sms = 148;
   double omega = 6.283185307179586476925286766559;  // 2*pi, TracerAndVorticityDistributions.f90:34-35
   double delta[3] = {0.0, 0.0, 0.05};               // ACTIVE, VERTEX, PASSIVE (smooth, :27)
-  tcb::PairCfg cfg64{256, 2, 256};
+  tcb::PairCfg cfg64{128, 6, 256};
   tcb::PairCfg cfg32{256, 4, 256};
   int var64 = 2, var32 = 0;  // pair-kernel variants in use (see kVariants64/32)
   bool auto32 = true;  // FP32C variant chosen per launch by problem size (tc_set_pair_variant turns it off)
-  bool auto64 = true;  // FP64: 32-source tiles for launches too small to fill a wave (likewise)
+  bool auto64 = true;  // FP64 variant chosen per launch by its size (likewise)
   int slots64_default = 0;  // resident CTAs per GPU of the default FP64 variant
-  int target_order = TC_ORDER_HILBERT;  // FP32C visiting order of targets
+  int target_order = TC_ORDER_HILBERT;  // visiting order of targets
   double adj_ms[3] = {0.0, 0.0, 0.0};  // last adjoint: forward sweep, recompute, backward
   int adj_mode = 6;  // adjoint VJP: 3-6 row pass, 0 two passes, 1 and 2 fused (tc_set_adjoint_mode)
   tcb::DevBuf order_buf[4];             // keys, sorted keys, indices, sort scratch
@@ -134,10 +134,11 @@ struct tc_ctx {
 };
 
 namespace tcb {
-// The automatic FP64 variants: the default, and the same shape with 32-source
-// tiles for launches that leave most of one wave's CTA slots empty.
+// The automatic FP64 variants: the default, and shapes with smaller target tiles for
+// launches over few sources or targets.
 constexpr int kAuto64Default = 2;
 constexpr int kAuto64Small = 6;
+constexpr int kAuto64Mid = 7;
 // Checked build: the extent the kernels check `site`'s indices against, n or the
 // cap tc_bounds_cap set (the smaller).
 inline long long bc_extent(const tc_ctx* ctx, int site, long long n) {
@@ -176,8 +177,9 @@ struct OrderJob {
   long long x_len, perm_len;
 };
 int compute_orders(tc_ctx* ctx, const OrderJob* jobs, int count);
-// Does a call visit its targets in that order?
-bool wants_order(const tc_ctx* ctx);
+// Does a call that evaluates `pairs` interactions, most_targets of its largest class's
+// targets, visit its targets in that order?
+bool wants_order(const tc_ctx* ctx, long long most_targets, double pairs);
 // Extents of an order computation: points in x, entries in perm, entries in each key and
 // index buffer.
 struct OrderExtents {
