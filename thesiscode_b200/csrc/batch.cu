@@ -419,7 +419,8 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
     if ((rc = tc_rk4_pack_sources(ctx))) return rc;  // autotuning ran stage-0 launches only
   }
   // the stage-0 epilogue's per-block kinetic-energy buffer: sized before any capture
-  if ((rc = R.keBlocks.ensure(((size_t)(B.nA_tot + B.nV_tot) + 255) / 256 * sizeof(double) + 16)))
+  if ((rc = R.keBlocks.ensure((size_t)tcb::epilogue_blocks_at_most(B.nA_tot + B.nV_tot) *
+                              sizeof(double))))
     return rc;
   if (nsteps > 0) {
     const std::vector<void*> ptrs = {R.x0A.ptr, R.z0.ptr, R.areaA.ptr, R.x0V.ptr, R.xiA.ptr,

@@ -460,19 +460,54 @@ int launch_pack(tc_ctx* ctx, const double* x, const double* zeta, const double* 
 // ---------------------------------------------------------------------------
 // Shared epilogue math.
 // ---------------------------------------------------------------------------
-// Sum of a partial row over the chunks; the checked build checks each read
-// against partial_len doubles (site: BC_EPI_PARTIAL or BC_STAGE_PARTIAL).
-__device__ __forceinline__ void reduce_row(const double* __restrict__ partial, int nchunks,
-                                           size_t n_out, size_t row, double T[3],
+// Rows and threads of an epilogue. A thread's chain of chunk loads is what an
+// epilogue over few rows takes its time with, so those rows are shared by kSplit
+// lanes each (level 4, 7,682 rows of 27 chunks: ten FP64 steps 2.19 -> 2.10 ms): a
+// warp takes 8 rows, lane l adds chunks l / 8, l / 8 + 4, ... of row l % 8, and the
+// lanes' sums are added pairwise. Rows enough to fill the GPU keep a thread each
+// (they are bound by memory).
+constexpr int kEpiThreads = 256;
+constexpr int kSplit = 4;
+constexpr int kSplitRows = 131072;  // rows up to which a row is shared
+constexpr int kRowsPerWarp = 32 / kSplit;
+
+static bool split_rows(int rows) { return rows <= kSplitRows; }
+static int epilogue_blocks(int rows) {
+  const int per_block = split_rows(rows) ? kEpiThreads / kSplit : kEpiThreads;
+  return std::max(1, (rows + per_block - 1) / per_block);
+}
+int epilogue_blocks_at_most(int rows) { return (rows + kEpiThreads / kSplit - 1) / (kEpiThreads / kSplit) + 1; }
+
+// Row of this thread and the first chunk it adds.
+template <bool SPLIT>
+__device__ __forceinline__ int epilogue_row(int* first) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  *first = SPLIT ? (threadIdx.x & 31) / kRowsPerWarp : 0;
+  return SPLIT ? (g >> 5) * kRowsPerWarp + g % kRowsPerWarp : g;
+}
+
+// Sum of a partial row over the chunks (all lanes of a warp call it; the result is
+// every lane's); the checked build checks each read against partial_len doubles
+// (site: BC_EPI_PARTIAL or BC_STAGE_PARTIAL).
+template <bool SPLIT>
+__device__ __forceinline__ void reduce_row(const double* __restrict__ partial, int first,
+                                           int nchunks, size_t n_out, size_t row, double T[3],
                                            BoundsRec* rec, int site, long long partial_len) {
   T[0] = T[1] = T[2] = 0.0;
-  for (int c = 0; c < nchunks; ++c) {
+#pragma unroll 4
+  for (int c = first; c < nchunks; c += SPLIT ? kSplit : 1) {
     const size_t o = (size_t)c * 3 * n_out + row;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const size_t j = o + (size_t)k * n_out;
       if (TC_BC(rec, site, j, partial_len)) T[k] += partial[j];
     }
+  }
+  if (SPLIT) {
+#pragma unroll
+    for (int o = kRowsPerWarp; o < 32; o <<= 1)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) T[k] += __shfl_xor_sync(0xffffffffu, T[k], o);
   }
 }
 
@@ -492,14 +527,19 @@ struct EpiBounds {
   long long x_len, perm_len, partial_len, out_len;
 };
 
-__global__ void velocity_epilogue_kernel(const double* __restrict__ x, const int* __restrict__ perm,
+template <bool SPLIT>
+__global__ void __launch_bounds__(kEpiThreads) velocity_epilogue_kernel(const double* __restrict__ x, const int* __restrict__ perm,
                                          int m, int i0, int i1, int row_offset, int n_out,
                                          int nchunks, const double* __restrict__ partial,
                                          double m2omega, double* __restrict__ dX,
                                          double* __restrict__ dVort, const EpiBounds eb) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= m) return;
-  const bool in_range = p >= i0 && p < i1;
+  int first;
+  const int p = epilogue_row<SPLIT>(&first);
+  const bool in_range = p < m && p >= i0 && p < i1;
+  double T[3];
+  reduce_row<SPLIT>(partial, first, in_range ? nchunks : 0, (size_t)n_out,
+                    (size_t)(row_offset + p), T, eb.rec, BC_EPI_PARTIAL, eb.partial_len);
+  if (p >= m || first != 0) return;
   int i = p;
   if (in_range && perm) {
     if (!TC_BC(eb.rec, BC_EPI_PERM, p, eb.perm_len)) return;
@@ -509,9 +549,6 @@ __global__ void velocity_epilogue_kernel(const double* __restrict__ x, const int
   if (in_range) {
     if (!TC_BC(eb.rec, BC_EPI_X, i, eb.x_len)) return;
     double xi[3] = {x[3 * (size_t)i], x[3 * (size_t)i + 1], x[3 * (size_t)i + 2]};
-    double T[3];
-    reduce_row(partial, nchunks, (size_t)n_out, (size_t)(row_offset + p), T, eb.rec,
-               BC_EPI_PARTIAL, eb.partial_len);
     velocity_from_sum(xi, T, u);
   }
   if (!TC_BC(eb.rec, BC_EPI_OUT, i, eb.out_len)) return;
@@ -531,7 +568,8 @@ int launch_velocity_epilogue(tc_ctx* ctx, const double* x, const int* perm, int 
   }
   const EpiBounds eb{ctx->bc_rec, bc_extent(ctx, BC_EPI_X, m), bc_extent(ctx, BC_EPI_PERM, m),
                      bc_extent(ctx, BC_EPI_PARTIAL, partial_len), bc_extent(ctx, BC_EPI_OUT, m)};
-  velocity_epilogue_kernel<<<(m + 255) / 256, 256, 0, ctx->stream>>>(
+  const auto kernel = split_rows(m) ? velocity_epilogue_kernel<true> : velocity_epilogue_kernel<false>;
+  kernel<<<epilogue_blocks(m), kEpiThreads, 0, ctx->stream>>>(
       x, perm, m, i0, i1, row_offset, n_out, nchunks, partial, -2.0 * ctx->omega, dX, dVort, eb);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
@@ -574,15 +612,16 @@ struct StageEpi {
   long long partial_len, chunks_len, keblock_len;
 };
 
-constexpr int kEpiThreads = 256;
-
+template <bool SPLIT>
 __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const StageEpi E) {
   __shared__ double red[kEpiThreads];
   const int lenA = E.a1 - E.a0, lenV = E.v1 - E.v0, lenQ = E.q1 - E.q0;
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  int first;
+  const int r = epilogue_row<SPLIT>(&first);
   double ke_area = 0.0;
-  if (r < lenA + lenV + lenQ) {
-    int cls, pos;
+  int cls = 0, pos = 0, row = 0, nch = 0;
+  const bool in = r < lenA + lenV + lenQ;
+  if (in) {
     if (r < lenA) {
       cls = 0;
       pos = E.a0 + r;
@@ -593,6 +632,15 @@ __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const Stage
       cls = 2;
       pos = E.q0 + (r - lenA - lenV);
     }
+    row = (cls == 0 ? 0 : cls == 1 ? E.nA : E.nA + E.nV) + pos;
+    nch = E.nchunks;
+    if (E.row_nchunks)
+      nch = TC_BC(E.rec, BC_STAGE_CHUNKS, row, E.chunks_len) ? E.row_nchunks[row] : 0;
+  }
+  double T[3];
+  reduce_row<SPLIT>(E.partial, first, nch, (size_t)E.n_out, (size_t)row, T, E.rec,
+                    BC_STAGE_PARTIAL, E.partial_len);
+  if (in && first == 0) {
     const int* perm = cls == 0 ? E.permA : cls == 1 ? E.permV : E.permQ;
     int i = pos;
     bool ok = true;
@@ -603,19 +651,13 @@ __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const Stage
     ok = ok && TC_BC(E.rec, BC_STAGE_STATE, i, E.state_len[cls]);
     if (cls == 0) ok = ok && TC_BC(E.rec, BC_STAGE_ACTIVE, i, E.active_len);
     if (ok) {
-      const int row = (cls == 0 ? 0 : cls == 1 ? E.nA : E.nA + E.nV) + pos;
       double* x0 = cls == 0 ? E.x0A : cls == 1 ? E.x0V : E.x0Q;
       double* xi = cls == 0 ? E.xiA : cls == 1 ? E.xiV : E.xiQ;
       double* nw = cls == 0 ? E.newA : cls == 1 ? E.newV : E.newQ;
       const double* xin = E.stage == 0 ? x0 : xi;
       const size_t b = 3 * (size_t)i;
       double xs[3] = {xin[b], xin[b + 1], xin[b + 2]};
-      double T[3], u[3];
-      int nch = E.nchunks;
-      if (E.row_nchunks)
-        nch = TC_BC(E.rec, BC_STAGE_CHUNKS, row, E.chunks_len) ? E.row_nchunks[row] : 0;
-      reduce_row(E.partial, nch, (size_t)E.n_out, (size_t)row, T, E.rec, BC_STAGE_PARTIAL,
-                 E.partial_len);
+      double u[3];
       velocity_from_sum(xs, T, u);
       if (cls == 0 && E.stage == 0) {
         double k2 = __dadd_rn(__dadd_rn(__dmul_rn(u[0], u[0]), __dmul_rn(u[1], u[1])),
@@ -763,14 +805,17 @@ int launch_stage_epilogue(tc_ctx* ctx, int stage, double dt, const int range[6],
   E.t_next = stage < 2 ? t_step + 0.5 * dt
                        : (stage == 2 ? t_step + dt : R.t0 + (double)(R.step + 1) * dt);
   const int rows = (E.a1 - E.a0) + (E.v1 - E.v0) + (E.q1 - E.q0);
-  const int blocks = std::max(1, (rows + kEpiThreads - 1) / kEpiThreads);
+  const int blocks = epilogue_blocks(rows);
   if (stage == 0) {
     int rc = R.keBlocks.ensure((size_t)blocks * sizeof(double));
     if (rc) return rc;
     E.keBlocks = R.keBlocks.as<double>();
   }
   E.keblock_len = bc_extent(ctx, BC_STAGE_KEBLOCK, cap_of<double>(R.keBlocks));
-  stage_epilogue_kernel<<<blocks, kEpiThreads, 0, ctx->stream>>>(E);
+  if (split_rows(rows))
+    stage_epilogue_kernel<true><<<blocks, kEpiThreads, 0, ctx->stream>>>(E);
+  else
+    stage_epilogue_kernel<false><<<blocks, kEpiThreads, 0, ctx->stream>>>(E);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
   if (stage == 0 && total_ke) {

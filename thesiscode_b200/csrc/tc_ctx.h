@@ -200,6 +200,8 @@ int launch_stage_epilogue(tc_ctx* ctx, int stage, double dt, const int range[6],
                           double* total_ke, const int* row_nchunks = nullptr,
                           const double* partial = nullptr, long long row_nchunks_len = 0,
                           long long partial_len = 0);
+// Blocks (and stage-0 kinetic-energy entries) of a stage epilogue over `rows` rows, at most.
+int epilogue_blocks_at_most(int rows);
 int resolve_slots(tc_ctx* ctx);
 // Checked build: points ctx->bc_rec at the device's violation record (allocated on first use
 // in each CUDA context).
