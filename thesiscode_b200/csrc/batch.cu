@@ -264,7 +264,7 @@ int enqueue_steps(tc_ctx* ctx, tc_batch_plan& B, double dt, int nsteps) {
 // shapes that were fastest on some workload of the level-7 sweep, all with the
 // default's accuracy (64-source FP32 flush; a 128-source flush is faster by
 // about 1% and raises the error by half).
-const int kTune32[] = {0, 1, 2, 3, 4, 5, 6, 7};
+const int kTune32[] = {0, 1, 2, 3, 4, 5, 6, 7, 12};
 const int kTune64[] = {2, 0, 1, 3, 6, 7};
 
 // Times one stage-0 launch of the whole batch (best of `reps`).

@@ -473,23 +473,31 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P)
 // Source pairing: the two f32x2 lanes of every FADD2/FFMA2/FMUL2 carry two
 // SOURCES (k, k+1) of one target, so a source tile sits in shared memory once
 // (no duplicated values): a warp-wide broadcast 128-bit shared load costs two
-// wavefronts of the SM-wide shared pipe, and a far source pair costs 7,
+// wavefronts of the SM-wide shared pipe, and a far source pair costs 6,
 // shared by the T targets of a thread.
 //
 // Two forms of the pair, chosen per 64-source segment (uniform over the CTA):
 // * near (11 FP32 operations): d = s_k - t_i, D = |d|^2 + e_i + e_k,
 //   T' += (2G_k / D) d;
-// * far (7 FP32 operations), for segments whose every source is farther than
+// * far (6 FP32 operations), for segments whose every source is farther than
 //   kFarRatio times the CTA's target radius rho (the largest |t_i|) from the
-//   origin: D/2 = A_k + B_i + s_k.(-t_i), A_k = (|s_k|^2 + e_k)/2 and
-//   B_i = (|t_i|^2 + e_i)/2 from FP64, and T' += r (G_k x'_k) with
-//   x'_k = R x_k (G x'_k from FP64, one rounding). In the rotated frame the
-//   first two coordinates of x'_k are small tangential offsets and the third
-//   is about 1, so the large common part of the sum (about sum r G) sits in
-//   the third coordinate only, and u_i = x_i x R^T T' multiplies it by the
-//   target's own small offset. With |s| > 3 rho, D >= (|s| - rho)^2 >=
-//   4|s|^2/9, so each rounding of the expansion costs at most a few ulps of D,
-//   as in the near form; the self pair never qualifies.
+//   origin. With a = -c.s_k and b = -c.t_i (minus the offsets' third coordinates,
+//   as e3 = c), the identity 1 - x_i.x_k = a + b - a b - s_x t_x - s_y t_y holds
+//   on and off the sphere for a unit origin c, so
+//       D/2 = a_k (1 - b_i) + (b_i + delta^2) - s_k,x t_i,x - s_k,y t_i,y
+//   takes 3 FMA with the targets' values in registers, a, b and b + delta^2 from
+//   FP64; and T' += r (G_k x'_k), x'_k = R x_k = (s_x, s_y, 1 - a) (G x' from FP64,
+//   one rounding). In the rotated frame the first two coordinates of x'_k are
+//   small tangential offsets and the third is about 1, so the large common part
+//   of the sum (about sum r G) sits in the third coordinate only, and u_i = x_i x
+//   R^T T' multiplies it by the target's own small offset. With |s| > 3 rho, D >=
+//   (|s| - rho)^2 >= 4|s|^2/9, so each rounding of the expansion costs at most a
+//   few ulps of D, as in the near form; the self pair never qualifies.
+// The far loop is bound by register reads: an FFMA2 of three register pairs takes
+// 3.4 cycles a warp and scheduler, 2.5 if the instruction before read one of them,
+// 2 only with two. So its instructions go operation by operation over the targets,
+// the source's pair staying in the operand cache. Level 7, a launch of 1.61e11 pairs:
+// 45.2 ms with 7 operations (the denominator from four products), 42.4 with 6.
 // Near and far sums go into the same accumulators: near sum w (x'_k - x'_i)
 // and far sum w x'_k differ by multiples of x'_i, which u = x_i x T ignores.
 //
@@ -555,16 +563,15 @@ __device__ __forceinline__ float combine_max(const unsigned* red) {
 template <int NT, int TS, int T = 1, bool SMACC = false, bool HILO = false>
 struct SpSmem {
   float4 a[TS / 2];        // (sx_k, sx_k+1, sy_k, sy_k+1)
-  float4 b[TS / 2];        // (sz_k, sz_k+1, A_k, A_k+1)
-  float4 c[TS / 2];        // (G x'_k, G x'_k+1, G y'_k, G y'_k+1)
-  float2 d[TS / 2];        // (G z'_k, G z'_k+1)
+  float4 b[TS / 2];        // (a_k, a_k+1, G x'_k, G x'_k+1)
+  float4 c[TS / 2];        // (G y'_k, G y'_k+1, G z'_k, G z'_k+1)
   float4 n[TS / 2];        // near form: (e_k, e_k+1, 2G_k, 2G_k+1)
   double frame[12];        // e1, e2, e3 (rows), origin c
   double csum[3][NT / 32]; // per-warp sums of the target positions
   double acc[SMACC ? 3 * T * NT : 1];  // FP64 accumulators [c][t][thread] (SMACC)
   float4 lo[HILO ? TS / 2 : 1];        // HILO: low parts (slx_k, slx_k+1, sly_k, sly_k+1)
-  float2 loz[HILO ? TS / 2 : 1];       // HILO: (slz_k, slz_k+1)
-  float tlo[HILO ? 3 * T * NT : 1];    // HILO: -(target low parts) [c][t][thread]
+  float2 loz[HILO ? TS / 2 : 1];       // HILO: low parts of (a_k, a_k+1)
+  float tlo[HILO ? 3 * T * NT : 1];    // HILO: low parts of (-t_x, -t_y, -b) [c][t][thread]
   unsigned tmin[NT / 32];
   unsigned rho[NT / 32];
 };
@@ -576,23 +583,26 @@ __device__ __forceinline__ float2 rcp2(float2 D) {
 // One far source pair against the thread's T targets.
 template <int T>
 __device__ __forceinline__ void sp_far_step(const float4 a, const float4 b, const float4 c,
-                                            const float2 d, const float2* ntx, const float2* nty,
-                                            const float2* ntz, const float2* bh, float2* fx,
-                                            float2* fy, float2* fz) {
+                                            const float2* ntx, const float2* nty, const float2* omb,
+                                            const float2* bd, float2* fx, float2* fy, float2* fz) {
   const float2 sx = make_float2(a.x, a.y), sy = make_float2(a.z, a.w);
-  const float2 sz = make_float2(b.x, b.y), ah = make_float2(b.z, b.w);
-  const float2 gx = make_float2(c.x, c.y), gy = make_float2(c.z, c.w);
+  const float2 ak = make_float2(b.x, b.y), gx = make_float2(b.z, b.w);
+  const float2 gy = make_float2(c.x, c.y), gz = make_float2(c.z, c.w);
+  float2 D[T];
 #pragma unroll
-  for (int t = 0; t < T; ++t) {
-    float2 D = __fadd2_rn(ah, bh[t]);
-    D = __ffma2_rn(sx, ntx[t], D);
-    D = __ffma2_rn(sy, nty[t], D);
-    D = __ffma2_rn(sz, ntz[t], D);
-    const float2 r = rcp2(D);
-    fx[t] = __ffma2_rn(r, gx, fx[t]);
-    fy[t] = __ffma2_rn(r, gy, fy[t]);
-    fz[t] = __ffma2_rn(r, d, fz[t]);
-  }
+  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(ak, omb[t], bd[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sx, ntx[t], D[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sy, nty[t], D[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) D[t] = rcp2(D[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) fx[t] = __ffma2_rn(D[t], gx, fx[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) fy[t] = __ffma2_rn(D[t], gy, fy[t]);
+#pragma unroll
+  for (int t = 0; t < T; ++t) fz[t] = __ffma2_rn(D[t], gz, fz[t]);
 }
 
 // FP64 accumulator of target t, coordinate c: a register, or (SMACC) a
@@ -622,59 +632,56 @@ struct SpAcc {
   }
 };
 
-// Converts the sources of the tile at ts into the CTA's frame: offsets s_k,
-// A_k = (|s_k|^2 + e_k)/2, G_k x'_k, e_k, 2G_k (and the hi/lo low parts),
-// padding past c1; records each warp's minimum |s_k|^2.
+// Converts the sources of the tile at ts into the CTA's frame: offsets s_k, a_k,
+// G_k x'_k, e_k, 2G_k (and the hi/lo low parts), padding past c1; records each
+// warp's minimum |s_k|^2.
 template <int NT, int TS, bool HILO, class Smem>
 __device__ __forceinline__ void sp_stage(const double4* __restrict__ src, int ts, int c1,
                                          const double* fr, Smem& sm, const UnitBounds& ub) {
   constexpr int NP = TS / 2;
   float smin = __int_as_float(0x7f800000);  // +inf
   for (int jp = threadIdx.x; jp < NP; jp += NT) {
-    float v[2][12];
+    float v[2][11];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int k = ts + 2 * jp + h;
-      // padding sources: zero weight, unit denominators
-      v[h][0] = v[h][1] = v[h][2] = 0.f;
-      v[h][3] = 1.f;
-      v[h][4] = v[h][5] = v[h][6] = 0.f;
-      v[h][7] = 1.f;
-      v[h][8] = 0.f;
-      v[h][9] = v[h][10] = v[h][11] = 0.f;
+      // padding sources: zero weight, denominators of about 1
+      v[h][0] = v[h][1] = 0.f;
+      v[h][2] = 1.f;
+      v[h][3] = v[h][4] = v[h][5] = 0.f;
+      v[h][6] = 1.f;
+      v[h][7] = 0.f;
+      v[h][8] = v[h][9] = v[h][10] = 0.f;
       if (k < c1 && TC_BC(ub.rec, BC_PAIR_SRC, k, ub.src_len)) {
         const double4 q = src[k];
         const double dx = q.x - fr[9], dy = q.y - fr[10], dz = q.z - fr[11];
         const double sxd = frame_dot(fr, dx, dy, dz), syd = frame_dot(fr + 3, dx, dy, dz),
-                     szd = frame_dot(fr + 6, dx, dy, dz);
-        const float sx = (float)sxd, sy = (float)syd, sz = (float)szd;
+                     akd = -frame_dot(fr + 6, dx, dy, dz);
+        const float sx = (float)sxd, sy = (float)syd, ak = (float)akd;
         if (HILO) {
-          v[h][9] = (float)(sxd - (double)sx);
-          v[h][10] = (float)(syd - (double)sy);
-          v[h][11] = (float)(szd - (double)sz);
+          v[h][8] = (float)(sxd - (double)sx);
+          v[h][9] = (float)(syd - (double)sy);
+          v[h][10] = (float)(akd - (double)ak);
         }
         const double ek = 1.0 - (q.x * q.x + q.y * q.y + q.z * q.z);
-        const float s2 = norm2_f32(sx, sy, sz);
-        smin = fminf(smin, s2);
+        smin = fminf(smin, norm2_f32(sx, sy, ak));
         v[h][0] = sx;
         v[h][1] = sy;
-        v[h][2] = sz;
-        v[h][3] = (float)(0.5 * ((double)s2 + ek));
-        v[h][4] = (float)(q.w * frame_dot(fr, q.x, q.y, q.z));
-        v[h][5] = (float)(q.w * frame_dot(fr + 3, q.x, q.y, q.z));
-        v[h][6] = (float)(q.w * frame_dot(fr + 6, q.x, q.y, q.z));
-        v[h][7] = (float)ek;
-        v[h][8] = (float)(2.0 * q.w);
+        v[h][2] = ak;
+        v[h][3] = (float)(q.w * sxd);
+        v[h][4] = (float)(q.w * syd);
+        v[h][5] = (float)fma(-q.w, akd, q.w);
+        v[h][6] = (float)ek;
+        v[h][7] = (float)(2.0 * q.w);
       }
     }
     sm.a[jp] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
     sm.b[jp] = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
     sm.c[jp] = make_float4(v[0][4], v[1][4], v[0][5], v[1][5]);
-    sm.d[jp] = make_float2(v[0][6], v[1][6]);
-    sm.n[jp] = make_float4(v[0][7], v[1][7], v[0][8], v[1][8]);
+    sm.n[jp] = make_float4(v[0][6], v[1][6], v[0][7], v[1][7]);
     if (HILO) {
-      sm.lo[jp] = make_float4(v[0][9], v[1][9], v[0][10], v[1][10]);
-      sm.loz[jp] = make_float2(v[0][11], v[1][11]);
+      sm.lo[jp] = make_float4(v[0][8], v[1][8], v[0][9], v[1][9]);
+      sm.loz[jp] = make_float2(v[0][10], v[1][10]);
     }
   }
   warp_store_min(smin, sm.tmin);
@@ -683,12 +690,12 @@ __device__ __forceinline__ void sp_stage(const double4* __restrict__ src, int ts
 // Far source pairs [j0, j1) of the staged tile against the thread's targets.
 template <int T, int UNROLL, class Smem>
 __device__ __forceinline__ void sp_far_run(const Smem& sm, int j0, int j1, const float2 (&ntx)[T],
-                                           const float2 (&nty)[T], const float2 (&ntz)[T],
-                                           const float2 (&bh)[T], float2 (&fx)[T], float2 (&fy)[T],
+                                           const float2 (&nty)[T], const float2 (&omb)[T],
+                                           const float2 (&bd)[T], float2 (&fx)[T], float2 (&fy)[T],
                                            float2 (&fz)[T]) {
 #pragma unroll UNROLL
   for (int j = j0; j < j1; ++j)
-    sp_far_step<T>(sm.a[j], sm.b[j], sm.c[j], sm.d[j], ntx, nty, ntz, bh, fx, fy, fz);
+    sp_far_step<T>(sm.a[j], sm.b[j], sm.c[j], ntx, nty, omb, bd, fx, fy, fz);
 }
 
 // Sums the staged tile into the thread's T targets: a tile whose
@@ -699,9 +706,9 @@ __device__ __forceinline__ void sp_far_run(const Smem& sm, int j0, int j1, const
 // otherwise one far test for the whole tile.
 template <int NT, int T, int TS, int FLUSH, int UNROLL, bool SMACC, bool HILO, int FARK, class Smem>
 __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
-                                       const float2 (&nty)[T], const float2 (&ntz)[T],
-                                       const float2 (&bh)[T], const float (&ei)[T],
-                                       float2 (&fx)[T], float2 (&fy)[T], float2 (&fz)[T],
+                                       const float2 (&nty)[T], const float2 (&omb)[T],
+                                       const float2 (&bd)[T], const float (&nb)[T],
+                                       const float (&ei)[T], float2 (&fx)[T], float2 (&fy)[T], float2 (&fz)[T],
                                        SpAcc<NT, T, SMACC>& acc) {
   constexpr int NP = TS / 2;
   constexpr int FP = FLUSH / 2;
@@ -711,7 +718,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
   const bool tile_far = combine_min<NT / 32>(sm.tmin) > lim;
   if (tile_far) {
     for (int jf = 0; jf < NP; jf += FPF) {
-      sp_far_run<T, UNROLL>(sm, jf, jf + FPF, ntx, nty, ntz, bh, fx, fy, fz);
+      sp_far_run<T, UNROLL>(sm, jf, jf + FPF, ntx, nty, omb, bd, fx, fy, fz);
 #pragma unroll
       for (int t = 0; t < T; ++t) {
         acc.add(0, t, (double)__fadd_rn(fx[t].x, fx[t].y));
@@ -725,7 +732,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
   for (int jf = 0; jf < NP; jf += FP) {
     const bool far = PERSEG && __uint_as_float(sm.tmin[jf / FP]) > lim;
     if (far) {
-      sp_far_run<T, UNROLL>(sm, jf, jf + FP, ntx, nty, ntz, bh, fx, fy, fz);
+      sp_far_run<T, UNROLL>(sm, jf, jf + FP, ntx, nty, omb, bd, fx, fy, fz);
     } else {
       // HILO: d = (s_hi - t_hi) + (s_lo - t_lo), accurate to a few ulps of d itself
       float ntl[HILO ? 3 * T : 1];
@@ -739,7 +746,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
         const float4 b = sm.b[j];
         const float4 n = sm.n[j];
         const float2 sx = make_float2(a.x, a.y), sy = make_float2(a.z, a.w);
-        const float2 sz = make_float2(b.x, b.y);
+        const float2 ak = make_float2(b.x, b.y);
         const float2 ee = make_float2(n.x, n.y), gg = make_float2(n.z, n.w);
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f);
         float2 loz = make_float2(0.f, 0.f);
@@ -751,7 +758,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
         for (int t = 0; t < T; ++t) {
           float2 dx = __fadd2_rn(sx, ntx[t]);
           float2 dy = __fadd2_rn(sy, nty[t]);
-          float2 dz = __fadd2_rn(sz, ntz[t]);
+          float2 dz = __fadd2_rn(ak, make_float2(nb[t], nb[t]));  // -(s_z - t_z)
           if (HILO) {
             dx = __fadd2_rn(dx, __fadd2_rn(make_float2(lo.x, lo.y), make_float2(ntl[t], ntl[t])));
             dy = __fadd2_rn(dy, __fadd2_rn(make_float2(lo.z, lo.w), make_float2(ntl[T + t], ntl[T + t])));
@@ -768,11 +775,12 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
         }
       }
     }
+    const float zsign = far ? 1.f : -1.f;
 #pragma unroll
     for (int t = 0; t < T; ++t) {
       acc.add(0, t, (double)__fadd_rn(fx[t].x, fx[t].y));
       acc.add(1, t, (double)__fadd_rn(fy[t].x, fy[t].y));
-      acc.add(2, t, (double)__fadd_rn(fz[t].x, fz[t].y));
+      acc.add(2, t, (double)(zsign * __fadd_rn(fz[t].x, fz[t].y)));
       fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
     }
   }
@@ -804,7 +812,7 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
   };
   // Origin: the CTA's targets' centroid, projected to the sphere (a smaller
   // patch radius than any one target gives: fewer near tiles, smaller FP32
-  // offsets); the middle target when the targets surround the centre.
+  // offsets); the middle target's direction when the targets surround the centre.
   double px = 0.0, py = 0.0, pz = 0.0;
 #pragma unroll
   for (int t = 0; t < T; ++t) {
@@ -838,18 +846,22 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
     }
     const double count = (double)min(TB, i_end - tile0);
     const double n2 = sx * sx + sy * sy + sz * sz;
-    double cx, cy, cz;
-    if (n2 > 0.25 * count * count) {
-      const double inv = 1.0 / sqrt(n2);
-      cx = sx * inv;
-      cy = sy * inv;
-      cz = sz * inv;
-    } else {
+    double cx = sx, cy = sy, cz = sz, m2 = n2;
+    if (!(n2 > 0.25 * count * count)) {
       const int c = TC_BC(ub.rec, BC_PAIR_X, mid, ub.x_len) ? mid : 0;
       cx = x[3 * (size_t)c];
       cy = x[3 * (size_t)c + 1];
       cz = x[3 * (size_t)c + 2];
+      m2 = cx * cx + cy * cy + cz * cz;
+      if (!(m2 > 1e-6 && m2 < 1e6)) {  // not finite or far off the sphere: any unit origin serves
+        cx = cy = 0.0;
+        cz = m2 = 1.0;
+      }
     }
+    const double inv = 1.0 / sqrt(m2);
+    cx *= inv;
+    cy *= inv;
+    cz *= inv;
     make_frame(cx, cy, cz, sm.frame);
     sm.frame[9] = cx;
     sm.frame[10] = cy;
@@ -859,8 +871,8 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
   const double* fr = sm.frame;
   const double cx = fr[9], cy = fr[10], cz = fr[11];
 
-  float2 ntx[T], nty[T], ntz[T], bh[T];
-  float ei[T];  // near form only: paired on use
+  float2 ntx[T], nty[T], omb[T], bd[T];  // -t_x, -t_y, 1 - b, b + delta^2
+  float nb[T], ei[T];  // near form only, paired on use: -b, e
   float2 fx[T], fy[T], fz[T];
   SpAcc<NT, T, SMACC> acc;
   acc.init(sm.acc);
@@ -872,22 +884,22 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
     const double px = x[3 * (size_t)ld], py = x[3 * (size_t)ld + 1], pz = x[3 * (size_t)ld + 2];
     const double dx = px - cx, dy = py - cy, dz = pz - cz;
     const double txd = frame_dot(fr, dx, dy, dz), tyd = frame_dot(fr + 3, dx, dy, dz),
-                 tzd = frame_dot(fr + 6, dx, dy, dz);
-    const float tx = (float)txd, ty = (float)tyd, tz = (float)tzd;
+                 bid = -frame_dot(fr + 6, dx, dy, dz);
+    const float tx = (float)txd, ty = (float)tyd, b = (float)bid;
     if (HILO) {
       sm.tlo[(0 * T + t) * NT + threadIdx.x] = -(float)(txd - (double)tx);
       sm.tlo[(1 * T + t) * NT + threadIdx.x] = -(float)(tyd - (double)ty);
-      sm.tlo[(2 * T + t) * NT + threadIdx.x] = -(float)(tzd - (double)tz);
+      sm.tlo[(2 * T + t) * NT + threadIdx.x] = -(float)(bid - (double)b);
     }
     const double E = (1.0 - (px * px + py * py + pz * pz)) + 2.0 * d2;
+    const float om = (float)(1.0 - bid), bdf = (float)(bid + d2);
     ntx[t] = make_float2(-tx, -tx);
     nty[t] = make_float2(-ty, -ty);
-    ntz[t] = make_float2(-tz, -tz);
+    omb[t] = make_float2(om, om);
+    bd[t] = make_float2(bdf, bdf);
+    nb[t] = -b;
     ei[t] = (float)E + kSelfBias;
-    const float t2 = norm2_f32(tx, ty, tz);
-    const float b = (float)(0.5 * ((double)t2 + E));
-    bh[t] = make_float2(b, b);
-    rho2 = fmaxf(rho2, t2);
+    rho2 = fmaxf(rho2, norm2_f32(tx, ty, b));
     fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
   }
   warp_store_max(rho2, sm.rho);
@@ -895,7 +907,8 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
     __syncthreads();
     sp_stage<NT, TS, HILO>(src, ts, c1, fr, sm, ub);
     __syncthreads();
-    sp_sum<NT, T, TS, FLUSH, UNROLL, SMACC, HILO, FARK>(sm, ntx, nty, ntz, bh, ei, fx, fy, fz, acc);
+    sp_sum<NT, T, TS, FLUSH, UNROLL, SMACC, HILO, FARK>(sm, ntx, nty, omb, bd, nb, ei, fx,
+                                                        fy, fz, acc);
   }
   // back to the global frame: T = R^T T'
 #pragma unroll

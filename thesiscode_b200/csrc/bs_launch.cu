@@ -49,13 +49,13 @@ template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64b(int g, cudaStream_t s, const BatchLaunch& B) {
   pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT><<<g, NT, 0, s>>>(B);
 }
-template <int NT, int T, int FLUSH, int MINB, int UNROLL, int FM>
+template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32b(int g, cudaStream_t s, const BatchLaunch& B) {
-  pair_fp32c_batch_kernel<NT, T, kTS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(B);
+  pair_fp32c_batch_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(B);
 }
-template <int NT, int T, int FLUSH, int MINB, int UNROLL, int FM>
+template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
-  pair_fp32c_kernel<NT, T, kTS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(P);
+  pair_fp32c_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(P);
 }
 
 #define V64(NT, TPT, MINB, UNROLL, SHORT, STRICT)                                            \
@@ -64,13 +64,15 @@ void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
                 (const void*)pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>,     \
                 launch64b<NT, TPT, MINB, UNROLL, SHORT, STRICT>,                              \
                 (const void*)pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, 0 }
-// FP32C: T targets per thread, FP32 flush every FLUSH sources, form bits FM
-#define V32(NT, T, FLUSH, MINB, UNROLL, FM)                                            \
-  PairVariant { TC_FP32C, NT, T, kTS, FLUSH, MINB, UNROLL,                             \
-                launch32<NT, T, FLUSH, MINB, UNROLL, FM>,                              \
-                (const void*)pair_fp32c_kernel<NT, T, kTS, FLUSH, MINB, UNROLL, FM>,   \
-                launch32b<NT, T, FLUSH, MINB, UNROLL, FM>,                             \
-                (const void*)pair_fp32c_batch_kernel<NT, T, kTS, FLUSH, MINB, UNROLL, FM>, FM }
+// FP32C: T targets per thread, source tiles of TS, FP32 flush every FLUSH sources,
+// form bits FM
+#define V32T(NT, T, TS, FLUSH, MINB, UNROLL, FM)                                         \
+  PairVariant { TC_FP32C, NT, T, TS, FLUSH, MINB, UNROLL,                                \
+                launch32<NT, T, TS, FLUSH, MINB, UNROLL, FM>,                            \
+                (const void*)pair_fp32c_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM>,      \
+                launch32b<NT, T, TS, FLUSH, MINB, UNROLL, FM>,                           \
+                (const void*)pair_fp32c_batch_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM>, FM }
+#define V32(NT, T, FLUSH, MINB, UNROLL, FM) V32T(NT, T, kTS, FLUSH, MINB, UNROLL, FM)
 
 // FP64: the `flush` field records the denominator mode (1 = fused, 0 =
 // rounded exactly like the reference).
@@ -92,15 +94,16 @@ static_assert(kAuto64Default == 2 && kAuto64Small == 6 && kAuto64Mid == 7,
 // 256 / 512 = tiles whose every source is far flushed every 2 / 4 flush
 // lengths.
 const PairVariant kVariants32[] = {
-    // 0: default from 131,072 sources (3 targets per thread); 1: default below (2 per thread)
-    V32(128, 3, 64, 6, 4, 8 | 2 | 256), V32(128, 2, 64, 6, 4, 8 | 512),
-    // 2-7: the batch autotuner's other candidates (4: the 64-source far flush of 0)
-    V32(128, 2, 64, 6, 4, 8 | 2 | 512), V32(128, 2, 64, 6, 4, 8 | 2 | 256),
+    // 0, 1, 12: chosen by the number of sources (use_fp32c_variant)
+    V32(128, 3, 64, 4, 4, 8 | 256), V32T(64, 3, 128, 64, 8, 4, 8 | 256),
+    // 2-7: the batch autotuner's other candidates
+    V32(128, 2, 64, 6, 4, 8 | 512), V32(128, 2, 64, 6, 4, 8 | 2 | 256),
     V32(128, 3, 64, 6, 4, 8 | 2), V32(128, 2, 64, 6, 4, 8), V32(128, 2, 64, 6, 4, 8 | 2),
-    V32(128, 3, 64, 6, 2, 8 | 2),
+    V32(128, 3, 64, 6, 4, 8 | 2 | 256),
     // 8-11: near tiles with hi/lo offsets (1e-7 at coarser grids, at a fraction of the speed)
     V32(128, 3, 64, 6, 4, 8 | 4 | 2), V32(128, 2, 64, 6, 4, 8 | 4), V32(128, 2, 64, 6, 4, 8 | 4 | 2),
     V32(128, 3, 64, 5, 4, 8 | 4 | 2),
+    V32(128, 2, 64, 6, 4, 8 | 2 | 512),
 };
 constexpr int kN64 = sizeof(kVariants64) / sizeof(kVariants64[0]);
 constexpr int kN32 = sizeof(kVariants32) / sizeof(kVariants32[0]);
@@ -133,20 +136,21 @@ int select_variant(tc_ctx* ctx, int precision, int id) {
   return TC_OK;
 }
 
-// Automatic FP32C variant: below kAutoSmallSources sources (icosahedral level
-// 6 and coarser) two targets per thread (variant 1: more CTAs for few
-// tiles, and smaller tile patches, hence smaller FP32 offsets), above it
-// three (variant 0: 2-4% faster from level 7 on); both flush all-far tiles
-// less often than mixed ones (0 every 128 sources, 1.8-2.0% faster than
-// every 64 at levels 7-8 with the same error; 1 every 256, 1.6% faster at
-// level 6, error 6.1e-8 against 5.2e-8 on the level-6 jet).
-constexpr int kAutoSmallSources = 131072;
-constexpr int kAutoSmallVariant = 1;
-constexpr int kAutoLargeVariant = 0;
+// Automatic FP32C variant. From 131,072 sources three targets a thread, all-far tiles
+// flushed every 128 sources; below, two, every 256 (more CTAs, and smaller tile
+// patches, hence fewer near tiles and smaller FP32 offsets); below 12,288 tiles of 192
+// targets and 128 sources, because on coarse grids the near form takes most of the
+// time and the far test's reach is three patch radii. Pair launches, ms (192 / 256 /
+// 384 targets a tile): level 4 refined 0.045 / 0.051 / -, level 5 0.228 / 0.224 / -,
+// level 6 refined 5.35 / 5.05 / 5.36, level 7 - / 41.4 / 41.0.
+constexpr int kAutoFewSources = 12288, kAutoMidSources = 131072;
+constexpr int kAutoFewVariant = 1, kAutoMidVariant = 12, kAutoLargeVariant = 0;
 
 int use_fp32c_variant(tc_ctx* ctx, int n) {
   if (!ctx->auto32) return TC_OK;
-  const int want = n < kAutoSmallSources ? kAutoSmallVariant : kAutoLargeVariant;
+  const int want = n < kAutoFewSources   ? kAutoFewVariant
+                   : n < kAutoMidSources ? kAutoMidVariant
+                                         : kAutoLargeVariant;
   return want == ctx->var32 ? TC_OK : select_variant(ctx, TC_FP32C, want);
 }
 
@@ -184,32 +188,32 @@ static int choose_chunks(int tiles, int n, int ts, int slots, int min_chunk, int
   return best;
 }
 
-constexpr int kFullWarps = 12;
+// Source chunk length of a launch of a few waves at most, by a model of its time. The
+// CTAs of one chunk walk len sources each; an SM holds `resident` of them at a time
+// and needs full_warps warps for its pipe's full rate, so a round of c CTAs takes
+// len x max(c, enough) (enough CTAs for that many warps) and, for its prologue,
+// epilogue and staging, about as long as kRoundSources more. Chunks are multiples of
+// gran sources. Level 4 (7,682 targets in tiles of 128): 27 chunks of 192.
 constexpr int kRoundSources = 64;
 
-// Source chunk length of an FP64 launch, by a model of its time. The CTAs of one
-// chunk walk len sources each; an SM holds `resident` of them at a time and needs
-// kFullWarps warps for the FP64 pipe's full rate, so a round of c CTAs takes len x
-// max(c, enough) (enough CTAs for that many warps) and, for its prologue, epilogue
-// and staging, about as long as kRoundSources more. Chunks are multiples of gran.
-static int fine_chunk_len(int tiles, int n, int num_sms, int slots, int warps, int max_chunks,
-                          int gran) {
+static int fine_chunk_len(int tiles, int n, int num_sms, int slots, int warps, int full_warps,
+                          int max_chunks, int gran) {
   const int resident = std::max(1, slots / num_sms);
-  const int enough = std::max(1, std::min(resident, kFullWarps / warps));
+  const int enough = std::max(1, std::min(resident, full_warps / warps));
   double best_cost = -1.0;
-  int best_len = n;
-  for (int s = 1; s <= max_chunks; ++s) {
-    int len = (n + s - 1) / s;
-    len = (len + gran - 1) / gran * gran;
-    const int chunks = (n + len - 1) / len;
-    const long long per_sm = ((long long)tiles * chunks + num_sms - 1) / num_sms;
-    const long long full = per_sm / resident, rest = per_sm % resident;
-    const double load = (double)full * resident + (rest ? std::max<long long>(rest, enough) : 0);
-    const double cost = load * len + (double)kRoundSources * enough * (double)(full + (rest ? 1 : 0));
+  int best_len = (n + gran - 1) / gran * gran;
+  // per_sm CTAs an SM: of the chunk counts that give as many, the largest has the shortest chunks
+  for (int per_sm = (tiles + num_sms - 1) / num_sms; per_sm <= 4 * resident; ++per_sm) {
+    const int s = std::min(max_chunks, per_sm * num_sms / tiles);
+    const int len = ((n + s - 1) / s + gran - 1) / gran * gran;
+    const int full = per_sm / resident, rest = per_sm % resident;
+    const double load = full * resident + (rest ? std::max(rest, enough) : 0);
+    const double cost = load * len + (double)kRoundSources * enough * (full + (rest ? 1 : 0));
     if (best_cost < 0.0 || cost < best_cost * 0.995) {
       best_cost = cost;
       best_len = len;
     }
+    if (s == max_chunks || len == gran) break;  // no shorter chunks
   }
   return best_len;
 }
@@ -227,23 +231,48 @@ static int count_tiles(const SegDesc* segs, int nseg, int tb) {
   return tiles;
 }
 
-// Automatic FP64 variant. The default's tiles of 768 targets leave SMs idle when
-// its whole-tile chunks fill less than 90% of one wave, and on coarse grids they
-// reach past the frame form's limit and cut the work into too few pieces: below
-// 12,288 sources tiles of 128 targets are faster (pair launch at levels 3 / 4 / 4
-// refined to 6,023: 12.6 / 43 / 55 us, tiles of 384: 11.2 / 49 / 63), below 65,536
-// tiles of 384 (level 5: 0.454 ms, of 128 0.496, of 768 0.49), from there on 768
-// (level 6: 6.41 ms, of 384 6.54).
-constexpr int kFewSources = 12288, kMidSources = 65536;
+// Chunk length of any launch. CTAs cost unequal times (near or far tiles, frame or
+// wide form), so a launch ends with a tail of about one CTA's length: chunks are cut
+// for kWaves waves, as far as they keep min_len sources (the prologue's share) and
+// their number kMostChunks (the epilogue's). FP32C level 6 refined in 4 / 8 / 24 / 48
+// chunks: 5.30 / 5.16 / 5.06 / 5.04 ms, level 7 in 1 / 4 / 16 / 24: 44.0 / 41.6 / 41.0 /
+// 40.8; FP64 level 5 in 8 / 24 / 48: 0.604 / 0.474 / 0.436 ms. Launches that stay below
+// three waves that way fill whole waves instead (choose_chunks), or, with the shapes
+// for few sources, minimise the model's time.
+constexpr int kWaves = 32;
 
-static int auto64_variant(const tc_ctx* ctx, const SegDesc* segs, int nseg, int n, int max_chunks) {
-  const PairVariant& v = kVariants64[kAuto64Default];
-  const int tiles = count_tiles(segs, nseg, v.nt * v.tpt);
-  const int slots = ctx->slots64_default;
-  const int len = whole_chunk_len(tiles, n, kTS, slots, ctx->min_chunk, max_chunks);
-  const long long items = (long long)tiles * ((n + len - 1) / len);
-  if (items * 10 < 9LL * slots || n < kFewSources) return kAuto64Small;
-  return n < kMidSources ? kAuto64Mid : kAuto64Default;
+static int chunk_length(const tc_ctx* ctx, const PairCfg& cfg, int slots, int tiles, int n,
+                        int max_chunks) {
+  const bool fp64 = ctx->precision == TC_FP64;
+  const int min_len = fp64 ? 448 : 768, most = std::min(max_chunks, fp64 ? 48 : 24);
+  const long long S = std::min<long long>(
+      {((long long)kWaves * slots + tiles - 1) / tiles, n / min_len, (long long)most});
+  const int gran = fp64 && ctx->var64 >= kAuto64Small ? 16 : cfg.ts;
+  if (S * tiles >= 3LL * slots) {
+    const int len = std::max(gran, (int)(n / S) / gran * gran);  // one chunk more, if there is room
+    return (n + len - 1) / len <= max_chunks ? len : len + gran;
+  }
+  const bool few = fp64 ? ctx->auto64 : ctx->auto32 && ctx->var32 == kAutoFewVariant;
+  if (few)
+    return fine_chunk_len(tiles, n, ctx->num_sms, slots, cfg.nt / 32, fp64 ? 12 : 16, max_chunks,
+                          gran);
+  return whole_chunk_len(tiles, n, cfg.ts, slots, ctx->min_chunk, max_chunks);
+}
+
+// Automatic FP64 variant: below 12,288 sources tiles of 128 targets are fastest (pair
+// launch at level 4 / level 4 refined to 6,023 panels: 43 / 55 us, tiles of 384 49 /
+// 63): on coarse grids larger tiles reach past the frame form's limit and cut the work
+// into too few pieces. Below 65,536 tiles of 384 are (level 5: 0.454 ms, of 128 0.496,
+// of 768 0.49), from there on 768 (level 6: 6.41 ms, of 384 6.54). Few targets take the
+// smaller tiles whatever the sources' number, or they would leave SMs idle (5,000
+// against level 6: 0.354 ms, in tiles of 768 0.477).
+constexpr int kFewSources = 12288, kMidSources = 65536;
+constexpr int kFewTargets = 6144, kMidTargets = 24576;
+
+static int auto64_variant(const SegDesc* segs, int nseg, int n) {
+  const int targets = count_tiles(segs, nseg, 1);
+  if (n < kFewSources || targets < kFewTargets) return kAuto64Small;
+  return n < kMidSources || targets < kMidTargets ? kAuto64Mid : kAuto64Default;
 }
 
 // A tile of 1/8 of the sphere's targets has a radius of about 0.7 at best, the
@@ -260,7 +289,7 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
     if (rc0) return rc0;
   }
   if (fp64 && ctx->auto64 && n > 0 && count_tiles(segs, nseg, 1) > 0) {
-    const int want = auto64_variant(ctx, segs, nseg, n, max_chunks);
+    const int want = auto64_variant(segs, nseg, n);
     if (want != ctx->var64) {
       const int rc = select_variant(ctx, TC_FP64, want);
       if (rc) return rc;
@@ -291,11 +320,7 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
   *grid = dim3(tiles, 0);
   if (tiles == 0 || n <= 0) return TC_OK;
   const int slots = fp64 ? ctx->slots64 : ctx->slots32;
-  const int chunk_len =
-      (fp64 && ctx->auto64)
-          ? fine_chunk_len(tiles, n, ctx->num_sms, slots, cur.nt / 32, max_chunks,
-                           ctx->var64 == kAuto64Default ? cur.ts : 16)
-          : whole_chunk_len(tiles, n, cur.ts, slots, ctx->min_chunk, max_chunks);
+  const int chunk_len = chunk_length(ctx, cur, slots, tiles, n, max_chunks);
   const int S = (n + chunk_len - 1) / chunk_len;
   P->src = src;
   P->n = n;
@@ -331,12 +356,20 @@ static int run_pairs(tc_ctx* ctx, const PairLaunch& P, dim3 grid) {
   return TC_OK;
 }
 
+// Chunks a launch may have: ctx->max_chunks, or for few rows up to kManyChunks as far as
+// their partial sums stay small (a few hundred targets against many sources).
+static int most_chunks(const tc_ctx* ctx, int n_out) {
+  constexpr size_t kManyChunks = 256, kManyBytes = size_t(64) << 20;
+  const size_t fit = kManyBytes / (3 * (size_t)std::max(n_out, 1) * sizeof(double));
+  return std::max(ctx->max_chunks, (int)std::min(kManyChunks, fit));
+}
+
 int launch_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4* src, int n,
                  long long src_len, int n_out, int* nchunks) {
   *nchunks = 0;
   PairLaunch P;
   dim3 grid;
-  int rc = plan_pairs(ctx, segs, nseg, src, n, src_len, n_out, ctx->max_chunks, &P, &grid);
+  int rc = plan_pairs(ctx, segs, nseg, src, n, src_len, n_out, most_chunks(ctx, n_out), &P, &grid);
   if (rc || grid.y == 0) return rc;
   if ((rc = ctx->partial.ensure((size_t)grid.y * 3 * (size_t)n_out * sizeof(double)))) return rc;
   P.partial = ctx->partial.as<double>();
@@ -355,8 +388,9 @@ int launch_pairs_into(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
   PairLaunch P;
   dim3 grid;
   int rc = plan_pairs(ctx, segs, nseg, src, n, src_len, n_out,
-                      (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)ctx->max_chunks)), &P,
-                      &grid);
+                      (int)std::max<size_t>(
+                          1, std::min<size_t>(fit, (size_t)most_chunks(ctx, n_out))),
+                      &P, &grid);
   if (rc || grid.y == 0) return rc;
   if ((size_t)grid.y * per_chunk > partial_bytes) {
     tc_record_error("pair partial sums need %zu bytes, %zu given", (size_t)grid.y * per_chunk,

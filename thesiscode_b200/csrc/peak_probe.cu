@@ -17,20 +17,19 @@ namespace {
 constexpr int kChains = 8;
 
 // The far-form pair step of the FP32C kernel itself (tcb::sp_far_run: per
-// source pair and target one FADD2, six FFMA2 and two MUFU reciprocals, the
-// source pair read from shared memory) with the default variant's shape:
-// 128 threads, 3 targets per thread, 6 CTAs per SM, 4 source pairs per
+// source pair and target six FFMA2 and two MUFU reciprocals, the source pair
+// read from shared memory) with the default variant's shape:
+// 128 threads, 3 targets per thread, 4 CTAs per SM, 4 source pairs per
 // unrolled body. The 128 source pairs stay resident in shared memory. There
 // is no staging, no far test, no flush and no near tile, so its rate
 // (pairs/s, one pair = one target x one source) is the ceiling of the pair
 // loop's instruction mix on this GPU.
-constexpr int kFarT = 3, kFarNT = 128, kFarNP = 128, kFarMinB = 6;
+constexpr int kFarT = 3, kFarNT = 128, kFarNP = 128, kFarMinB = 4;
 
 struct FarTile {
   float4 a[kFarNP];
   float4 b[kFarNP];
   float4 c[kFarNP];
-  float2 d[kFarNP];
 };
 
 __global__ void __launch_bounds__(kFarNT, kFarMinB) probe_far_pairs(int iters, float b, float c,
@@ -38,24 +37,23 @@ __global__ void __launch_bounds__(kFarNT, kFarMinB) probe_far_pairs(int iters, f
   __shared__ FarTile tile;
   for (int j = threadIdx.x; j < kFarNP; j += kFarNT) {
     const float s = 1e-3f * (float)(j + 1);
-    tile.a[j] = make_float4(s, -s, 0.5f * s, 0.25f * s);         // offsets x, y of two sources
-    tile.b[j] = make_float4(-s, s, 1.0f + s, 1.0f + 2.0f * s);   // offsets z; A_k near 1
-    tile.c[j] = make_float4(b * s, c * s, s, -s);                // G x', G y'
-    tile.d[j] = make_float2(s, 2.0f * s);                        // G z'
+    tile.a[j] = make_float4(s, -s, 0.5f * s, 0.25f * s);              // offsets x, y of two sources
+    tile.b[j] = make_float4(1.0f + s, 1.0f + 2.0f * s, b * s, c * s);  // a_k near 1; G x'
+    tile.c[j] = make_float4(s, -s, s, 2.0f * s);                      // G y', G z'
   }
   __syncthreads();
-  float2 ntx[kFarT], nty[kFarT], ntz[kFarT], bh[kFarT], fx[kFarT], fy[kFarT], fz[kFarT];
+  float2 ntx[kFarT], nty[kFarT], omb[kFarT], bd[kFarT], fx[kFarT], fy[kFarT], fz[kFarT];
 #pragma unroll
   for (int t = 0; t < kFarT; ++t) {
     const float u = 1e-4f * (float)(threadIdx.x + 32 * t);
     ntx[t] = make_float2(-u, -u);
     nty[t] = make_float2(u, u);
-    ntz[t] = make_float2(-0.5f * u, -0.5f * u);
-    bh[t] = make_float2(0.5f + u, 0.5f + u);
+    omb[t] = make_float2(1.0f - 0.5f * u, 1.0f - 0.5f * u);
+    bd[t] = make_float2(0.5f + u, 0.5f + u);
     fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
   }
   for (int i = 0; i < iters; ++i)
-    tcb::sp_far_run<kFarT, 4>(tile, 0, kFarNP, ntx, nty, ntz, bh, fx, fy, fz);
+    tcb::sp_far_run<kFarT, 4>(tile, 0, kFarNP, ntx, nty, omb, bd, fx, fy, fz);
   float s = 0.f;
 #pragma unroll
   for (int t = 0; t < kFarT; ++t) s += fx[t].x + fx[t].y + fy[t].x + fy[t].y + fz[t].x + fz[t].y;
