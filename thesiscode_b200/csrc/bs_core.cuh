@@ -421,7 +421,8 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
       // out with the multiple of x'_i = (t_1, t_2, 1 - b_i), then back: T = R^T T'
       const double* fr = sm.frame;
       const double v0 = -tg[t][0], v1 = -tg[t][1], v2 = tg[t][2];
-      const double lam = fma(T[0], v0, fma(T[1], v1, T[2] * v2)) / fma(v0, v0, fma(v1, v1, v2 * v2));
+      const double lam = fma(T[0], v0, fma(T[1], v1, T[2] * v2)) *
+                         rcp_f64(fma(v0, v0, fma(v1, v1, v2 * v2)));
       const double a0 = fma(-lam, v0, T[0]), a1 = fma(-lam, v1, T[1]), a2 = fma(-lam, v2, T[2]);
 #pragma unroll
       for (int c = 0; c < 3; ++c) T[c] = fma(fr[c], a0, fma(fr[3 + c], a1, fr[6 + c] * a2));
