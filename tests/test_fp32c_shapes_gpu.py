@@ -58,3 +58,37 @@ def test_automatic_shapes(gpu):
             got.append(v.value)
         ctx.close()
     assert got == [1, 12, 12, 12, 12, 0, 0, 0, 6, 7, 7, 2, 2, 2, 7, 6]
+
+
+@pytest.mark.parametrize("n,m", [(700, 5000), (131072, 1500)])
+def test_a_bad_target_spoils_its_own_row_only(gpu, n, m):
+    """Device arrays are not scanned. A NaN or infinite target shares its thread's reciprocals with
+    another target and must not reach it: every other row stays within twice the bound of the
+    rows without it (its CTA takes another origin, so they round differently)."""
+    import torch
+
+    w = configs.gaussian(level=7 if n > 100000 else 4, delta=0.02)
+    x, a = w.xA[:n].copy(), w.areaA[:n].copy()
+    rng = np.random.default_rng(8)
+    z = rng.standard_normal(n)
+    X = np.ascontiguousarray(configs.gaussian(level=5, delta=0.02).xV[:m])
+    ctx = Context(0, "fp32c")
+    ctx.set_deltas(0.02, 0.02, 0.02)
+    out = []
+    for bad in (False, True):
+        Y = X.copy()
+        if bad:
+            Y[1234] = np.nan
+            Y[400, 1] = np.inf
+        dev = [torch.from_numpy(v).cuda() for v in (Y, x, z, a)]
+        u = torch.zeros((m, 3), dtype=torch.float64, device="cuda")
+        p = [ctypes.c_void_p(t.data_ptr()) for t in dev + [u]]
+        N.call("tc_bs_velocity_device", ctx.handle, N.TC_VERTEX, p[0], m, p[1], p[2], p[3], n, 0, m, p[4], None)
+        torch.cuda.synchronize()
+        out.append(u.cpu().numpy())
+    ctx.close()
+    fine = np.ones(m, bool)
+    fine[[1234, 400]] = False
+    assert np.all(np.isnan(out[1][~fine]).any(axis=1)) and np.all(np.isfinite(out[1][fine]))
+    tol = 4.0 * 2.0 ** -24 / (0.6 * np.sqrt(4.0 * np.pi / w.nA))
+    assert np.abs(out[1][fine] - out[0][fine]).max() <= 2.0 * tol * np.abs(out[0]).max()

@@ -90,16 +90,17 @@ const PairVariant kVariants64[] = {
 static_assert(kAuto64Default == 2 && kAuto64Small == 6 && kAuto64Mid == 7,
               "automatic FP64 variants");
 // FP32C form bits (SpForm in bs_core.cuh): 8 = source-paired form (all
-// variants), 2 = FP64 accumulators in shared memory, 4 = hi/lo near offsets,
+// variants), 2 = FP64 accumulators in shared memory, 4 = hi/lo near offsets, 16 =
+// two targets share reciprocals in every second far source pair,
 // 256 / 512 = tiles whose every source is far flushed every 2 / 4 flush
 // lengths.
 const PairVariant kVariants32[] = {
     // 0, 1, 12: chosen by the number of sources (use_fp32c_variant)
-    V32(128, 3, 64, 4, 4, 8 | 256), V32T(64, 3, 128, 64, 8, 4, 8 | 256),
+    V32(128, 3, 64, 4, 4, 8 | 16 | 256), V32T(64, 3, 128, 64, 8, 4, 8 | 16 | 256),
     // 2-7: the batch autotuner's other candidates
     V32(128, 2, 64, 6, 4, 8 | 512), V32(128, 2, 64, 6, 4, 8 | 2 | 256),
     V32(128, 3, 64, 6, 4, 8 | 2), V32(128, 2, 64, 6, 4, 8), V32(128, 2, 64, 6, 4, 8 | 2),
-    V32(128, 3, 64, 6, 4, 8 | 2 | 256),
+    V32(128, 3, 64, 6, 4, 8 | 2 | 16 | 256),
     // 8-11: near tiles with hi/lo offsets (1e-7 at coarser grids, at a fraction of the speed)
     V32(128, 3, 64, 6, 4, 8 | 4 | 2), V32(128, 2, 64, 6, 4, 8 | 4), V32(128, 2, 64, 6, 4, 8 | 4 | 2),
     V32(128, 3, 64, 5, 4, 8 | 4 | 2),

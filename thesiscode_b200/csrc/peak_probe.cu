@@ -17,8 +17,8 @@ namespace {
 constexpr int kChains = 8;
 
 // The far-form pair step of the FP32C kernel itself (tcb::sp_far_run: per
-// source pair and target six FFMA2 and two MUFU reciprocals, the source pair
-// read from shared memory) with the default variant's shape:
+// source pair and three targets 18 FFMA2 and six MUFU reciprocals, or 21 and four
+// in every second source pair, which comes from shared memory) with the default variant's shape:
 // 128 threads, 3 targets per thread, 4 CTAs per SM, 4 source pairs per
 // unrolled body. The 128 source pairs stay resident in shared memory. There
 // is no staging, no far test, no flush and no near tile, so its rate
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(kFarNT, kFarMinB) probe_far_pairs(int iters, f
     fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
   }
   for (int i = 0; i < iters; ++i)
-    tcb::sp_far_run<kFarT, 4>(tile, 0, kFarNP, ntx, nty, omb, bd, fx, fy, fz);
+    tcb::sp_far_run<kFarT, 4, true>(tile, 0, kFarNP, ntx, nty, omb, bd, fx, fy, fz);
   float s = 0.f;
 #pragma unroll
   for (int t = 0; t < kFarT; ++t) s += fx[t].x + fx[t].y + fy[t].x + fy[t].y + fz[t].x + fz[t].y;

@@ -42,7 +42,7 @@ struct PairVariant {
   const void* fn;
   void (*launch_batch)(int grid, cudaStream_t stream, const BatchLaunch& B);
   const void* fn_batch;
-  int form;  // FP32C: bit 3 source-paired form (every variant), bit 1 shared-memory FP64 accumulators, bit 2 hi/lo near offsets, bits 8-9 log2 of flush lengths per flush in all-far tiles. FP64: 0
+  int form;  // FP32C: bit 3 source-paired form (every variant), bit 1 shared-memory FP64 accumulators, bit 2 hi/lo near offsets, bit 4 shared far reciprocals, bits 8-9 log2 of flush lengths per flush in all-far tiles. FP64: 0
 };
 
 // Target segment as the host describes it before tiles are assigned.
