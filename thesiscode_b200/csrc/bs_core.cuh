@@ -22,6 +22,13 @@ namespace tcb {
 
 constexpr int kNoSelf = INT32_MIN;
 
+// Start of a kernel launched by launch_chained: everything before it in the stream is
+// done when this returns, and the next chained kernel may be set up meanwhile.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 struct TargetSeg {
   const double* x;  // targets, x[3*i + c]
   const int* perm;  // target at position p in [i0,i1) is perm[p] (null: p itself)
@@ -439,6 +446,7 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
 
 template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P) {
+  chain_begin();
   __shared__ Fp64Smem<NT, TPT, TS> sm;
   const TargetSeg& G = find_seg(P, blockIdx.x);
   const int tile0 = G.i0 + (int)(blockIdx.x - G.tile_begin) * (NT * TPT);
@@ -970,6 +978,7 @@ struct SpForm {
 
 template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 __global__ void __launch_bounds__(NT, MINB) pair_fp32c_kernel(const PairLaunch P) {
+  chain_begin();
   using F = SpForm<FM>;
   const TargetSeg& G = find_seg(P, blockIdx.x);
   const int tile0 = G.i0 + (int)(blockIdx.x - G.tile_begin) * (NT * T);
@@ -1034,6 +1043,7 @@ __device__ __forceinline__ int next_item(int* counter, int* slot) {
 
 template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 __global__ void __launch_bounds__(NT, MINB) pair_fp32c_batch_kernel(const BatchLaunch B) {
+  chain_begin();
   using F = SpForm<FM>;
   __shared__ int slot;
   __shared__ SpSmem<NT, TS, T, F::smacc, F::hilo> sm;
@@ -1051,6 +1061,7 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp32c_batch_kernel(const BatchL
 
 template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_batch_kernel(const BatchLaunch B) {
+  chain_begin();
   __shared__ Fp64Smem<NT, TPT, TS> sm;
   __shared__ int slot;
   for (int it = next_item(B.counter, &slot); it < B.n_items; it = next_item(B.counter, &slot)) {

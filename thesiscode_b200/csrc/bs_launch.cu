@@ -43,19 +43,19 @@ constexpr int kTS = 256;
 
 template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64(dim3 g, cudaStream_t s, const PairLaunch& P) {
-  pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT><<<g, NT, 0, s>>>(P);
+  launch_chained(pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, dim3(g), dim3(NT), 0, s, P);
 }
 template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64b(int g, cudaStream_t s, const BatchLaunch& B) {
-  pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT><<<g, NT, 0, s>>>(B);
+  launch_chained(pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, dim3(g), dim3(NT), 0, s, B);
 }
 template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32b(int g, cudaStream_t s, const BatchLaunch& B) {
-  pair_fp32c_batch_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(B);
+  launch_chained(pair_fp32c_batch_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM>, dim3(g), dim3(NT), 0, s, B);
 }
 template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
-  pair_fp32c_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM><<<g, NT, 0, s>>>(P);
+  launch_chained(pair_fp32c_kernel<NT, T, TS, FLUSH, MINB, UNROLL, FM>, dim3(g), dim3(NT), 0, s, P);
 }
 
 #define V64(NT, TPT, MINB, UNROLL, SHORT, STRICT)                                            \
@@ -418,6 +418,7 @@ struct PackBounds {
 __global__ void pack_kernel(const double* __restrict__ x, const double* __restrict__ zeta,
                             const double* __restrict__ area, int n, double4* __restrict__ out,
                             const PackBounds pb) {
+  chain_begin();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   if (!TC_BC(pb.rec, BC_PACK_IN, k, pb.in_len)) return;
@@ -432,6 +433,7 @@ __global__ void pack_strat_kernel(const double* __restrict__ x, const double* __
                                   const double* __restrict__ area, int n, double two_omega,
                                   double t, double* __restrict__ zeta, double4* __restrict__ out,
                                   const PackBounds pb) {
+  chain_begin();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   if (!TC_BC(pb.rec, BC_PACK_IN, k, pb.in_len)) return;
@@ -463,8 +465,8 @@ int launch_pack_strat(tc_ctx* ctx, double t) {
       (long long)std::min(R.z0.bytes / sizeof(double), R.src.bytes / sizeof(double4));
   const PackBounds pb{ctx->bc_rec, bc_extent(ctx, BC_PACK_IN, in_len),
                       bc_extent(ctx, BC_PACK_OUT, out_len)};
-  pack_strat_kernel<<<(R.nA + 255) / 256, 256, 0, ctx->stream>>>(
-      R.x0A.as<double>(), R.absA.as<double>(), R.areaA.as<double>(), R.nA, 2.0 * ctx->omega, t,
+  launch_chained(
+      pack_strat_kernel, dim3((R.nA + 255) / 256), dim3(256), 0, ctx->stream, R.x0A.as<double>(), R.absA.as<double>(), R.areaA.as<double>(), R.nA, 2.0 * ctx->omega, t,
       R.z0.as<double>(), R.src.as<double4>(), pb);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
@@ -487,7 +489,8 @@ int launch_pack(tc_ctx* ctx, const double* x, const double* zeta, const double* 
   if (n <= 0) return TC_OK;
   const PackBounds pb{ctx->bc_rec, bc_extent(ctx, BC_PACK_IN, n),
                       bc_extent(ctx, BC_PACK_OUT, out_len)};
-  pack_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(x, zeta, area, n, out, pb);
+  launch_chained(pack_kernel, dim3((n + 255) / 256), dim3(256), 0, ctx->stream, x, zeta, area, n,
+                 out, pb);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
   return TC_OK;
@@ -569,6 +572,7 @@ __global__ void __launch_bounds__(kEpiThreads) velocity_epilogue_kernel(const do
                                          int nchunks, const double* __restrict__ partial,
                                          double m2omega, double* __restrict__ dX,
                                          double* __restrict__ dVort, const EpiBounds eb) {
+  chain_begin();
   int first;
   const int p = epilogue_row<SPLIT>(&first);
   const bool in_range = p < m && p >= i0 && p < i1;
@@ -605,8 +609,8 @@ int launch_velocity_epilogue(tc_ctx* ctx, const double* x, const int* perm, int 
   const EpiBounds eb{ctx->bc_rec, bc_extent(ctx, BC_EPI_X, m), bc_extent(ctx, BC_EPI_PERM, m),
                      bc_extent(ctx, BC_EPI_PARTIAL, partial_len), bc_extent(ctx, BC_EPI_OUT, m)};
   const auto kernel = split_rows(m) ? velocity_epilogue_kernel<true> : velocity_epilogue_kernel<false>;
-  kernel<<<epilogue_blocks(m), kEpiThreads, 0, ctx->stream>>>(
-      x, perm, m, i0, i1, row_offset, n_out, nchunks, partial, -2.0 * ctx->omega, dX, dVort, eb);
+  launch_chained(
+      kernel, dim3(epilogue_blocks(m)), dim3(kEpiThreads), 0, ctx->stream, x, perm, m, i0, i1, row_offset, n_out, nchunks, partial, -2.0 * ctx->omega, dX, dVort, eb);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
   return TC_OK;
@@ -650,6 +654,7 @@ struct StageEpi {
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const StageEpi E) {
+  chain_begin();
   __shared__ double red[kEpiThreads];
   const int lenA = E.a1 - E.a0, lenV = E.v1 - E.v0, lenQ = E.q1 - E.q0;
   int first;
@@ -758,6 +763,7 @@ __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const Stage
 
 __global__ void ke_finalize_kernel(const double* __restrict__ blocks, int nblocks,
                                    double* __restrict__ out) {
+  chain_begin();
   __shared__ double red[256];
   double s = 0.0;
   for (int j = threadIdx.x; j < nblocks; j += 256) s += blocks[j];
@@ -848,14 +854,13 @@ int launch_stage_epilogue(tc_ctx* ctx, int stage, double dt, const int range[6],
     E.keBlocks = R.keBlocks.as<double>();
   }
   E.keblock_len = bc_extent(ctx, BC_STAGE_KEBLOCK, cap_of<double>(R.keBlocks));
-  if (split_rows(rows))
-    stage_epilogue_kernel<true><<<blocks, kEpiThreads, 0, ctx->stream>>>(E);
-  else
-    stage_epilogue_kernel<false><<<blocks, kEpiThreads, 0, ctx->stream>>>(E);
+  launch_chained(split_rows(rows) ? stage_epilogue_kernel<true> : stage_epilogue_kernel<false>,
+                 dim3(blocks), dim3(kEpiThreads), 0, ctx->stream, E);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 1;
   if (stage == 0 && total_ke) {
-    ke_finalize_kernel<<<1, 256, 0, ctx->stream>>>(E.keBlocks, blocks, total_ke);
+    launch_chained(ke_finalize_kernel, dim3(1), dim3(256), 0, ctx->stream, E.keBlocks, blocks,
+                   total_ke);
     TC_CUDA_TRY(cudaGetLastError());
     ctx->launches += 1;
   }

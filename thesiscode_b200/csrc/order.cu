@@ -57,6 +57,7 @@ constexpr int kOrderCells = 1 << kOrderCellBits;
 constexpr int kOrderShift = kSphereKeyBits - kOrderCellBits;
 
 __global__ void small_keys_kernel(const SmallOrders P) {
+  chain_begin();
   const SmallOrder& S = P.s[blockIdx.y];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= S.n) return;
@@ -72,6 +73,7 @@ __global__ void small_keys_kernel(const SmallOrders P) {
 // is not used, so the result is deterministic. A cell that holds most points
 // (all targets in one spot) costs n^2 / 1024 comparisons a thread, 2.6e5 at most.
 __global__ void __launch_bounds__(kOrderThreads) small_order_kernel(const SmallOrders P) {
+  chain_begin();
   extern __shared__ unsigned order_smem[];
   const SmallOrder& S = P.s[blockIdx.x];
   unsigned* keys = order_smem;                                       // n
@@ -141,9 +143,9 @@ int launch_small_orders(tc_ctx* ctx, const SmallOrders& P, int count) {
   const size_t smem = small_order_smem(most);
   TC_CUDA_TRY(cudaFuncSetAttribute(small_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)small_order_smem(kSmallOrder)));
-  small_keys_kernel<<<dim3((most + 127) / 128, count), 128, 0, ctx->stream>>>(P);
+  launch_chained(small_keys_kernel, dim3((most + 127) / 128, count), dim3(128), 0, ctx->stream, P);
   TC_CUDA_TRY(cudaGetLastError());
-  small_order_kernel<<<count, kOrderThreads, smem, ctx->stream>>>(P);
+  launch_chained(small_order_kernel, dim3(count), dim3(kOrderThreads), smem, ctx->stream, P);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 2;
   return TC_OK;

@@ -12,6 +12,28 @@
 
 namespace tcb {
 
+// Launch of a kernel that begins with chain_begin(): its CTAs may be set up while the
+// kernel before it in the stream still runs, so that the gap between dependent
+// kernels, most of a small call's time, shrinks. A sum from device arrays, without and
+// with: level 3 panels FP64 19.6 and 15.7 us, FP32C 24.7 and 18.0, level 4 panels 40.1
+// and 33.7, 42.1 and 33.0. Replayed from a CUDA graph the steps take the same time
+// either way.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // A growable device allocation owned by the context.
 struct DevBuf {
   void* ptr = nullptr;
