@@ -288,7 +288,16 @@ __global__ void __launch_bounds__(kFNT) adj_fused_kernel(const AdjFused P) {
 // r <- r + r (1 - D r) of 2 FMA each (2 steps: full FP64; 1 step: the seed's
 // error squared). TPT rows per thread share each source's shared-memory loads.
 // No reduction across threads. Rows: partial[(chunk*9 + c)*n + i].
-constexpr int kRNT = 128, kRTS = 128, kRowSums = 9;
+//
+// The pass is bound by the FP64 pipe and its register reads: 19 of the 22 operations
+// are FMA of three registers, one of which (the source's) two rows share, 2.7 cycles
+// on average, so 6.5e11 pairs/s is its bound at two rows. CTAs of 64 threads and 24
+// chunks (128 and 7 before) keep the last round short: the row pass and its small
+// kernels, level 5 0.795 -> 0.755 ms, level 6 11.0 -> 10.45; three or four rows a
+// thread came to 0.763 to 0.83 and 10.4 to 10.7. (The explicit minimum of one CTA an SM
+// lets the compiler use 138 registers; at the 122 it takes without, level 6 takes 11.1.)
+constexpr int kRNT = 64, kRTS = 128, kRowSums = 9;
+constexpr int kRowChunks = 24, kRowMinChunk = 192;
 
 struct RowLaunch {
   const double4* ra;  // {x, y, z, G x} per panel
@@ -349,7 +358,8 @@ __device__ __forceinline__ void adj_row_source(const double4 q, const double4 w,
 }
 
 template <int TPT, int NEWTON, int UNROLL>
-__global__ void __launch_bounds__(kRNT) adj_row_kernel(const RowLaunch P) {
+__global__ void __launch_bounds__(kRNT, 1) adj_row_kernel(const RowLaunch P) {
+  chain_begin();
   __shared__ double4 sa[kRTS];  // {x_j, G_j x_j}
   __shared__ double4 sb[kRTS];  // {G_j y_j, G_j z_j, v_j,x, v_j,y}
   __shared__ double sc[kRTS];   // v_j,z
@@ -412,39 +422,68 @@ __global__ void __launch_bounds__(kRNT) adj_row_kernel(const RowLaunch P) {
   }
 }
 
+// What a stage's cotangent g = J(Y_s)^T (dt lk_s) goes to: acc += g, and the cotangent
+// of the stage before, lk_{s-1} = b l' + c g (none for the first stage). Buffers
+// [3n | n].
+struct AdjNext {
+  double* acc;
+  double* lk;         // null: first stage
+  const double* lam;  // l'
+  double b, c;
+};
+
+__device__ __forceinline__ void adj_next(const AdjNext& N, size_t j, double g) {
+  N.acc[j] += g;
+  if (N.lk) N.lk[j] = fma(N.c, g, N.b * N.lam[j]);
+}
+
 // Row-pass combination: g_x = -(S1 x ut + C + G P)/(4 pi), g_zeta = -A (x . P)/(4 pi),
-// from `chunks` partial blocks of kRowSums rows each, added in chunk order.
-__global__ void adj_combine_row_kernel(const double* __restrict__ x, const double* __restrict__ ut,
-                                       const double* __restrict__ zeta,
-                                       const double* __restrict__ area, int n,
-                                       const double* __restrict__ p, int chunks,
-                                       double* __restrict__ out_x, double* __restrict__ out_z,
-                                       BoundsRec* bc, long long p_len) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// from `chunks` partial blocks of kRowSums rows each. Four lanes share a row (lane l
+// of a warp adds chunks l / 8, l / 8 + 4, ... of row l % 8; level 5, 24 chunks), as the
+// chain of loads of one thread would take longest. The stage's axpby updates are part
+// of it: three launches a stage less, level 5 0.755 -> 0.731 ms a product, level 4
+// 0.118 -> 0.092.
+__global__ void __launch_bounds__(256) adj_combine_row_kernel(
+    const double* __restrict__ x, const double* __restrict__ ut, const double* __restrict__ zeta,
+    const double* __restrict__ area, int n, const double* __restrict__ p, int chunks,
+    const AdjNext next, BoundsRec* bc, long long p_len) {
+  chain_begin();
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (g >> 5) * 8 + (g & 7), first = (threadIdx.x & 31) >> 3;
   const size_t N = (size_t)n, b = 3 * (size_t)i;
   double s[kRowSums];
 #pragma unroll
   for (int w = 0; w < kRowSums; ++w) s[w] = 0.0;
-  for (int c = 0; c < chunks; ++c)
+  if (i < n) {
+#pragma unroll 2
+    for (int c = first; c < chunks; c += 4)
 #pragma unroll
-    for (int w = 0; w < kRowSums; ++w) {
-      const size_t j = ((size_t)c * kRowSums + w) * N + i;
-      if (TC_BC(bc, BC_ADJ_COMBINE, j, p_len)) s[w] += p[j];
-    }
+      for (int w = 0; w < kRowSums; ++w) {
+        const size_t j = ((size_t)c * kRowSums + w) * N + i;
+        if (TC_BC(bc, BC_ADJ_COMBINE, j, p_len)) s[w] += p[j];
+      }
+  }
+#pragma unroll
+  for (int w = 0; w < kRowSums; ++w) {
+    s[w] += __shfl_xor_sync(0xffffffffu, s[w], 8);
+    s[w] += __shfl_xor_sync(0xffffffffu, s[w], 16);
+  }
+  if (i >= n || first != 0) return;
   const double u0 = ut[b], u1 = ut[b + 1], u2 = ut[b + 2];
   const double G = zeta[i] * area[i];
   const double g0 = (s[1] * u2 - s[2] * u1) + s[3] + G * s[6];
   const double g1 = (s[2] * u0 - s[0] * u2) + s[4] + G * s[7];
   const double g2 = (s[0] * u1 - s[1] * u0) + s[5] + G * s[8];
   const double R = x[b] * s[6] + x[b + 1] * s[7] + x[b + 2] * s[8];
-  out_x[b] = -kInv4Pi * g0;
-  out_x[b + 1] = -kInv4Pi * g1;
-  out_x[b + 2] = -kInv4Pi * g2;
-  out_z[i] = -kInv4Pi * area[i] * R;
+  adj_next(next, b, -kInv4Pi * g0);
+  adj_next(next, b + 1, -kInv4Pi * g1);
+  adj_next(next, b + 2, -kInv4Pi * g2);
+  adj_next(next, 3 * N + i, -kInv4Pi * area[i] * R);
 }
 
 // v_i = ut_i x x_i with ut_i = mu_x,i + (-2 Omega mu_z,i) z_hat, mu = dt * l_k.
+// ROW: the row pass's inputs only (ra, rb, rc); otherwise the other passes' as well.
+template <bool ROW>
 __global__ void adj_prepare_kernel(const double* __restrict__ x, const double* __restrict__ lkx,
                                    const double* __restrict__ lkz, const double* __restrict__ zeta,
                                    const double* __restrict__ area, int n, double dt, double m2omega,
@@ -452,6 +491,7 @@ __global__ void adj_prepare_kernel(const double* __restrict__ x, const double* _
                                    double4* __restrict__ src1, double4* __restrict__ src2a,
                                    double2* __restrict__ src2b, double4* __restrict__ ra,
                                    double4* __restrict__ rb, double* __restrict__ rc) {
+  chain_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t b = 3 * (size_t)i;
@@ -462,26 +502,28 @@ __global__ void adj_prepare_kernel(const double* __restrict__ x, const double* _
   ut[b] = u0;
   ut[b + 1] = u1;
   ut[b + 2] = u2;
-  v[b] = v0;
-  v[b + 1] = v1;
-  v[b + 2] = v2;
   const double G = zeta[i] * area[i];
-  src1[i] = make_double4(x0, x1, x2, G);
-  src2a[i] = make_double4(x0, x1, x2, v0);
-  src2b[i] = make_double2(v1, v2);
+  if (!ROW) {
+    v[b] = v0;
+    v[b + 1] = v1;
+    v[b + 2] = v2;
+    src1[i] = make_double4(x0, x1, x2, G);
+    src2a[i] = make_double4(x0, x1, x2, v0);
+    src2b[i] = make_double2(v1, v2);
+  }
   ra[i] = make_double4(x0, x1, x2, G * x0);
   rb[i] = make_double4(G * x1, G * x2, v0, v1);
   rc[i] = v2;
 }
 
-// lY_i = J(Y)^T mu: gx (3 per row) and gz (1 per row), written to out_x/out_z.
+// lY_i = J(Y)^T mu: gx (3 per row) and gz (1 per row), added on by adj_next.
 // p1: chunks of `st1` rows each, the first 6 = (S1, S2); p2: chunks of `st2`
 // rows each, the first 7 = (P, Q, R).
 __global__ void adj_combine_kernel(const double* __restrict__ x, const double* __restrict__ ut,
                                    const double* __restrict__ zeta, const double* __restrict__ area,
                                    int n, const double* __restrict__ p1, int ch1, int st1,
                                    const double* __restrict__ p2, int ch2, int st2,
-                                   double* __restrict__ out_x, double* __restrict__ out_z) {
+                                   const AdjNext next) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t N = (size_t)n, b = 3 * (size_t)i;
@@ -496,18 +538,20 @@ __global__ void adj_combine_kernel(const double* __restrict__ x, const double* _
   const double g0 = (s[1] * u2 - s[2] * u1) + s[3] + G * (t[0] + t[3]);
   const double g1 = (s[2] * u0 - s[0] * u2) + s[4] + G * (t[1] + t[4]);
   const double g2 = (s[0] * u1 - s[1] * u0) + s[5] + G * (t[2] + t[5]);
-  out_x[b] = -kInv4Pi * g0;
-  out_x[b + 1] = -kInv4Pi * g1;
-  out_x[b + 2] = -kInv4Pi * g2;
-  out_z[i] = -kInv4Pi * area[i] * t[6];
+  adj_next(next, b, -kInv4Pi * g0);
+  adj_next(next, b + 1, -kInv4Pi * g1);
+  adj_next(next, b + 2, -kInv4Pi * g2);
+  adj_next(next, 3 * N + i, -kInv4Pi * area[i] * t[6]);
 }
 
-// Linear combinations of adjoint vectors: y = a*x + b*y (in place on y), n4 = 4*nA
-// values laid out as [3*nA positions | nA vorticities] in one buffer.
-__global__ void axpby_kernel(double a, const double* __restrict__ x, double b, double* __restrict__ y,
-                             size_t n) {
+// Start of a step's backward sweep: acc = l' (the identity part), lk_4 = b l'.
+__global__ void adj_begin_kernel(const double* __restrict__ lam, double b, double* __restrict__ acc,
+                                 double* __restrict__ lk, size_t n) {
+  chain_begin();
   size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (j < n) y[j] = a * x[j] + b * y[j];
+  if (j >= n) return;
+  acc[j] = lam[j];
+  lk[j] = b * lam[j];
 }
 
 }  // namespace
@@ -527,15 +571,16 @@ struct AdjWork {
 };
 
 int adj_stage_vjp(tc_ctx* ctx, AdjWork& W, const double* y, const double* lk, double dt,
-                  double* out) {
-  // y and lk, out: [3nA | nA] buffers
+                  const tcb::AdjNext& next) {
+  // y and lk: [3nA | nA] buffers
   const int n = W.nA;
   const double* yx = y;
   const double* yz = y + 3 * (size_t)n;
   const double* area = ctx->rk.areaA.as<double>();
   const int threads = 256, blocks = (n + threads - 1) / threads;
-  tcb::adj_prepare_kernel<<<blocks, threads, 0, ctx->stream>>>(
-      yx, lk, lk + 3 * (size_t)n, yz, area, n, dt, -2.0 * ctx->omega, W.ut.as<double>(),
+  tcb::launch_chained(
+      ctx->adj_mode >= 3 ? tcb::adj_prepare_kernel<true> : tcb::adj_prepare_kernel<false>,
+      dim3(blocks), dim3(threads), 0, ctx->stream, yx, lk, lk + 3 * (size_t)n, yz, area, n, dt, -2.0 * ctx->omega, W.ut.as<double>(),
       W.v.as<double>(), W.s1.as<double4>(), W.s2a.as<double4>(), W.s2b.as<double2>(),
       W.ra.as<double4>(), W.rb.as<double4>(), W.rc.as<double>());
   TC_CUDA_TRY(cudaGetLastError());
@@ -554,28 +599,13 @@ int adj_stage_vjp(tc_ctx* ctx, AdjWork& W, const double* y, const double* lk, do
     // thread, one Newton step
     const int tpt = mode == 7 ? 3 : (mode == 4 || mode == 6) ? 2 : 1;
     const int newton = mode <= 4 ? 2 : 1;
-    const void* fn = tpt == 3   ? (const void*)tcb::adj_row_kernel<3, 1, 1>
-                     : tpt == 1 ? (newton == 2 ? (const void*)tcb::adj_row_kernel<1, 2, 2>
-                                               : (const void*)tcb::adj_row_kernel<1, 1, 2>)
-                                : (newton == 2 ? (const void*)tcb::adj_row_kernel<2, 2, 1>
-                                               : (const void*)tcb::adj_row_kernel<2, 1, 1>);
+    void (*const kernel)(const tcb::RowLaunch) =
+        tpt == 3   ? tcb::adj_row_kernel<3, 1, 1>
+        : tpt == 1 ? (newton == 2 ? tcb::adj_row_kernel<1, 2, 2> : tcb::adj_row_kernel<1, 1, 2>)
+                   : (newton == 2 ? tcb::adj_row_kernel<2, 2, 2> : tcb::adj_row_kernel<2, 1, 2>);
     const int rows_per_cta = tcb::kRNT * tpt;
     const int tiles = (n + rows_per_cta - 1) / rows_per_cta;
-    int per_sm = 0;
-    TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, tcb::kRNT, 0));
-    const int slots = std::max(1, per_sm) * ctx->num_sms;
-    // whole waves: the chunk count that best fills tiles x chunks into the resident slots
-    S = 1;
-    double best = 0.0;
-    for (int c = 1; c <= 32; ++c) {
-      if (c > 1 && (n + c - 1) / c < 1024) break;
-      const long long items = (long long)tiles * c, waves = (items + slots - 1) / slots;
-      const double eff = (double)items / (double)(waves * slots);
-      if (eff > best + 0.02) {
-        best = eff;
-        S = c;
-      }
-    }
+    S = std::max(1, std::min(tcb::kRowChunks, n / tcb::kRowMinChunk));
     int chunk = (n + S - 1) / S;
     chunk = (chunk + tcb::kRTS - 1) / tcb::kRTS * tcb::kRTS;
     S = (n + chunk - 1) / chunk;
@@ -594,21 +624,11 @@ int adj_stage_vjp(tc_ctx* ctx, AdjWork& W, const double* y, const double* lk, do
                      tcb::bc_extent(ctx, tcb::BC_ADJ_ROW_IN, src_len),
                      tcb::bc_extent(ctx, tcb::BC_ADJ_ROW_OUT, p1_len)};
     const dim3 grid(tiles, S);
-    if (tpt == 3)
-      tcb::adj_row_kernel<3, 1, 1><<<grid, tcb::kRNT, 0, ctx->stream>>>(R);
-    else if (tpt == 1 && newton == 2)
-      tcb::adj_row_kernel<1, 2, 2><<<grid, tcb::kRNT, 0, ctx->stream>>>(R);
-    else if (tpt == 1)
-      tcb::adj_row_kernel<1, 1, 2><<<grid, tcb::kRNT, 0, ctx->stream>>>(R);
-    else if (newton == 2)
-      tcb::adj_row_kernel<2, 2, 1><<<grid, tcb::kRNT, 0, ctx->stream>>>(R);
-    else
-      tcb::adj_row_kernel<2, 1, 1><<<grid, tcb::kRNT, 0, ctx->stream>>>(R);
-    TC_CUDA_TRY(cudaGetLastError());
-    tcb::adj_combine_row_kernel<<<blocks, threads, 0, ctx->stream>>>(
-        yx, W.ut.as<double>(), yz, area, n, W.p1.as<double>(), S, out, out + 3 * (size_t)n,
-        ctx->bc_rec, tcb::bc_extent(ctx, tcb::BC_ADJ_COMBINE, p1_len));
-    TC_CUDA_TRY(cudaGetLastError());
+    TC_CUDA_TRY(tcb::launch_chained(kernel, grid, dim3(tcb::kRNT), 0, ctx->stream, R));
+    TC_CUDA_TRY(tcb::launch_chained(tcb::adj_combine_row_kernel, dim3((n + 63) / 64), dim3(256), 0,
+                                    ctx->stream, yx, W.ut.as<double>(), yz, area, n,
+                                    W.p1.as<double>(), S, next, ctx->bc_rec,
+                                    tcb::bc_extent(ctx, tcb::BC_ADJ_COMBINE, p1_len)));
     ctx->launches += 3;
     ctx->pair_launches += 1;
     ctx->pair_interactions += (long long)n * (long long)(n - 1);
@@ -659,16 +679,9 @@ int adj_stage_vjp(tc_ctx* ctx, AdjWork& W, const double* y, const double* lk, do
   }
   tcb::adj_combine_kernel<<<blocks, threads, 0, ctx->stream>>>(
       yx, W.ut.as<double>(), yz, area, n, W.p1.as<double>(), S, st1,
-      p2ptr ? p2ptr : W.p2.as<double>(), S2, st2, out, out + 3 * (size_t)n);
+      p2ptr ? p2ptr : W.p2.as<double>(), S2, st2, next);
   TC_CUDA_TRY(cudaGetLastError());
   ctx->launches += 2;
-  return TC_OK;
-}
-
-int axpby(tc_ctx* ctx, double a, const double* x, double b, double* y, size_t n) {
-  tcb::axpby_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(a, x, b, y, n);
-  TC_CUDA_TRY(cudaGetLastError());
-  ctx->launches += 1;
   return TC_OK;
 }
 
@@ -847,10 +860,6 @@ int adjoint_impl(tc_ctx* ctx, const double* xA0, const double* zetaA0, const dou
   // backward sweep, one checkpoint segment at a time
   double* lk = W.lk.as<double>();
   double* acc = W.tmp.as<double>();
-  double* ly = nullptr;
-  DevBuf lyb;
-  if ((rc = lyb.ensure(B))) return rc;
-  ly = lyb.as<double>();
   for (int seg = (nsteps - 1) / ckpt_every; seg >= 0 && nsteps > 0; --seg) {
     const int s0 = seg * ckpt_every, s1 = std::min(nsteps, s0 + ckpt_every);
     if (seg != last_seg) {
@@ -866,21 +875,17 @@ int adjoint_impl(tc_ctx* ctx, const double* xA0, const double* zetaA0, const dou
     }
     for (int step = s1 - 1; step >= s0; --step) {
       const double* Y = ys + (size_t)(step - s0) * 4 * W.n4;
-      // acc = l' (the identity part); lk for stage 4 = l'/6
-      TC_CUDA_TRY(cudaMemcpyAsync(acc, lam, B, cudaMemcpyDeviceToDevice, ctx->stream));
       const double bcoef[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
       const double ccoef[4] = {0.0, 0.5, 0.5, 1.0};  // Y_s = X + c_s k_{s-1}
-      // lk_4 = l'/6
-      if ((rc = axpby(ctx, bcoef[3], lam, 0.0, lk, W.n4))) return rc;
+      TC_CUDA_TRY(tcb::launch_chained(tcb::adj_begin_kernel, dim3((unsigned)((W.n4 + 255) / 256)),
+                                      dim3(256), 0, ctx->stream, lam, bcoef[3], acc, lk, W.n4));
+      ctx->launches += 1;
       for (int s = 3; s >= 0; --s) {
-        if ((rc = adj_stage_vjp(ctx, W, Y + (size_t)s * W.n4, lk, dt, ly))) return rc;
-        if ((rc = axpby(ctx, 1.0, ly, 1.0, acc, W.n4))) return rc;       // l += lY_s
-        if (s > 0) {                                                     // lk_{s-1} = b l' + c_s lY_s
-          if ((rc = axpby(ctx, bcoef[s - 1], lam, 0.0, lk, W.n4))) return rc;
-          if ((rc = axpby(ctx, ccoef[s], ly, 1.0, lk, W.n4))) return rc;
-        }
+        // l += lY_s, lk_{s-1} = b l' + c_s lY_s (the row pass has read lk_s by then)
+        const tcb::AdjNext next{acc, s > 0 ? lk : nullptr, lam, s > 0 ? bcoef[s - 1] : 0.0, ccoef[s]};
+        if ((rc = adj_stage_vjp(ctx, W, Y + (size_t)s * W.n4, lk, dt, next))) return rc;
       }
-      TC_CUDA_TRY(cudaMemcpyAsync(lam, acc, B, cudaMemcpyDeviceToDevice, ctx->stream));
+      std::swap(lam, acc);
     }
   }
   TC_CUDA_TRY(cudaEventRecord(ev[2], ctx->stream));
