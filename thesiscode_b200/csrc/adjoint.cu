@@ -29,6 +29,7 @@
 // checkpoint (one extra forward pass in total).
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <vector>
 
 #include "tc_ctx.h"
@@ -559,16 +560,34 @@ __global__ void adj_begin_kernel(const double* __restrict__ lam, double b, doubl
 
 using tcb::DevBuf;
 
-namespace {
-
-struct AdjWork {
+// The adjoint's buffers stay with the context between calls (to tc_reset_rk4 or
+// tc_destroy) while they are small: allocating and freeing a dozen takes milliseconds, as
+// long as the adjoint of a level-4 grid.
+struct tc_adjoint_work {
+  static constexpr size_t kKeepBytes = size_t(512) << 20;
   int nA = 0;
   size_t n4 = 0;
   DevBuf ck;        // checkpoints: ncheck x (3nA + nA)
   DevBuf ys;        // stage inputs of one segment: (steps*4) x (3nA + nA)
   DevBuf lam, lk, tmp;  // adjoint state, lk, accumulators (4nA each)
   DevBuf ut, v, s1, s2a, s2b, ra, rb, rc, p1, p2;
+  size_t bytes() const {
+    size_t b = 0;
+    for (const DevBuf* d : {&ck, &ys, &lam, &lk, &tmp, &ut, &v, &s1, &s2a, &s2b, &ra, &rb, &rc, &p1, &p2})
+      b += d->bytes;
+    return b;
+  }
 };
+
+void tc_adjoint_free(tc_ctx* ctx) {
+  delete ctx->adjoint;
+  ctx->adjoint = nullptr;
+}
+
+namespace {
+
+using AdjWork = tc_adjoint_work;
+
 
 int adj_stage_vjp(tc_ctx* ctx, AdjWork& W, const double* y, const double* lk, double dt,
                   const tcb::AdjNext& next) {
@@ -773,7 +792,15 @@ int adjoint_impl(tc_ctx* ctx, const double* xA0, const double* zetaA0, const dou
   }
   int rc = tc_rk4_load(ctx, xA0, zetaA0, areaA, nA, nullptr, 0, nullptr, 0, 0);
   if (rc) return rc;
-  AdjWork W;
+  if (!ctx->adjoint) ctx->adjoint = new (std::nothrow) tc_adjoint_work();
+  if (!ctx->adjoint) return TC_ERR_NOMEM;
+  struct KeepSmall {  // frees large buffers at the end of the call
+    tc_ctx* ctx;
+    ~KeepSmall() {
+      if (ctx->adjoint->bytes() > tc_adjoint_work::kKeepBytes) tc_adjoint_free(ctx);
+    }
+  } keep_small{ctx};
+  AdjWork& W = *ctx->adjoint;
   W.nA = nA;
   W.n4 = 4 * (size_t)nA;
   const size_t B = W.n4 * sizeof(double);

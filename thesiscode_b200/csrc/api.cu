@@ -92,6 +92,61 @@ int scan_results_status(tc_ctx* ctx, const HostArray* a, int count) {
   return TC_OK;
 }
 
+// Arrays that one kernel copies between the staging buffer and the device.
+struct StageCopy {
+  static constexpr int kMost = 6;
+  const double* from[kMost];
+  double* to[kMost];
+  size_t n[kMost];
+  int count = 0;
+};
+
+__global__ void stage_copy_kernel(const StageCopy C) {
+  tcb::chain_begin();
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (int a = 0; a < C.count; ++a)
+    for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < C.n[a]; j += stride)
+      C.to[a][j] = C.from[a][j];
+}
+
+// Whether the arrays of a call (`total` doubles) go through the staging buffer, which is
+// then free to be written: not on a stream under capture, whose replays would read what
+// the buffer holds by then.
+bool stage_ready(tc_ctx* ctx, size_t total) {
+  if (total == 0 || total * sizeof(double) > tcb::HostStage::kStageBytes) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  tcb::HostStage& S = ctx->stage;
+  if (!S.host) {
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, tcb::HostStage::kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||
+        cudaEventCreateWithFlags(&S.read, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      if (h) cudaFreeHost(h);
+      return false;  // no page-locked memory to be had: the arrays are copied one by one
+    }
+    S.host = static_cast<char*>(h);
+    S.dev = static_cast<char*>(d);
+    return true;
+  }
+  return cudaEventSynchronize(S.read) == cudaSuccess;
+}
+
+int stage_launch(tc_ctx* ctx, const StageCopy& C) {
+  size_t most = 1;
+  for (int a = 0; a < C.count; ++a) most = std::max(most, C.n[a]);
+  const int blocks = (int)std::min<size_t>((most + 255) / 256, (size_t)ctx->num_sms);
+  TC_CUDA_TRY(tcb::launch_chained(stage_copy_kernel, dim3(blocks), dim3(256), 0, ctx->stream, C));
+  TC_CUDA_TRY(cudaEventRecord(ctx->stage.read, ctx->stream));
+  ctx->launches += 1;
+  return TC_OK;
+}
+
 int begin(tc_ctx* ctx) {
   if (!ctx) {
     tc_record_error("null context");
@@ -207,10 +262,19 @@ extern "C" int tc_destroy(tc_ctx* ctx) {
   for (auto& b : ctx->order_buf) b.release();
   tc_batch_free(ctx);
   tc_advance_graph_free(ctx);
+  tc_adjoint_free(ctx);
+  ctx->stage.release();
   for (cudaEvent_t e : ctx->pair_events) cudaEventDestroy(e);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return TC_OK;
+}
+
+void tcb::HostStage::release() {
+  if (read) cudaEventDestroy(read);
+  if (host) cudaFreeHost(host);
+  host = dev = nullptr;
+  read = nullptr;
 }
 
 extern "C" int tc_set_stream(tc_ctx* ctx, void* stream) {
@@ -515,13 +579,26 @@ int rk4_load(tc_ctx* ctx, const double* xA, const double* zetaA, const double* a
   cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   const size_t D = sizeof(double);
   cudaStream_t s = ctx->stream;
-  if (nA) {
-    TC_CUDA_TRY(cudaMemcpyAsync(R.x0A.ptr, xA, 3 * (size_t)nA * D, kind, s));
-    TC_CUDA_TRY(cudaMemcpyAsync(R.z0.ptr, zetaA, (size_t)nA * D, kind, s));
-    TC_CUDA_TRY(cudaMemcpyAsync(R.areaA.ptr, areaA, (size_t)nA * D, kind, s));
+  const double* from[5] = {xA, zetaA, areaA, xV, xQ};
+  double* const to[5] = {R.x0A.as<double>(), R.z0.as<double>(), R.areaA.as<double>(),
+                         R.x0V.as<double>(), R.x0Q.as<double>()};
+  const size_t len[5] = {3 * (size_t)nA, (size_t)nA, (size_t)nA, 3 * (size_t)nV, 3 * (size_t)nQ};
+  if (!on_device && stage_ready(ctx, len[0] + len[1] + len[2] + len[3] + len[4])) {
+    StageCopy C;
+    size_t at = 0;
+    for (int a = 0; a < 5; ++a) {
+      if (len[a] == 0) continue;
+      memcpy(ctx->stage.host + at, from[a], len[a] * D);
+      C.from[C.count] = reinterpret_cast<const double*>(ctx->stage.dev + at);
+      C.to[C.count] = to[a];
+      C.n[C.count++] = len[a];
+      at += len[a] * D;
+    }
+    if ((rc = stage_launch(ctx, C))) return rc;
+  } else {
+    for (int a = 0; a < 5; ++a)
+      if (len[a]) TC_CUDA_TRY(cudaMemcpyAsync(to[a], from[a], len[a] * D, kind, s));
   }
-  if (nV) TC_CUDA_TRY(cudaMemcpyAsync(R.x0V.ptr, xV, 3 * (size_t)nV * D, kind, s));
-  if (nQ) TC_CUDA_TRY(cudaMemcpyAsync(R.x0Q.ptr, xQ, 3 * (size_t)nQ * D, kind, s));
   R.ready = true;
   R.ordered = false;
   R.strat = false;
@@ -537,6 +614,51 @@ extern "C" int tc_rk4_load(tc_ctx* ctx, const double* xA, const double* zetaA,
   return rk4_load(ctx, xA, zetaA, areaA, nA, xV, nV, xQ, nQ, on_device, true);
 }
 
+namespace {
+
+// The state, the kinetic energies and totalKE[nsteps] to host or device memory (null
+// arrays are left out); waits for host copies.
+int rk4_store(tc_ctx* ctx, double* xA, double* zetaA, double* xV, double* xQ, double* kineticEnergy,
+              double* totalKE, int nsteps, int on_device) {
+  tcb::Rk4State& R = ctx->rk;
+  cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+  const size_t D = sizeof(double);
+  cudaStream_t s = ctx->stream;
+  double* const to[6] = {xA, zetaA, xV, xQ, kineticEnergy, totalKE};
+  const double* from[6] = {R.x0A.as<double>(), R.z0.as<double>(), R.x0V.as<double>(),
+                           R.x0Q.as<double>(), R.ke.as<double>(), R.totalKE.as<double>()};
+  size_t len[6] = {3 * (size_t)R.nA, (size_t)R.nA, 3 * (size_t)R.nV, 3 * (size_t)R.nQ,
+                   (size_t)R.nA, (size_t)std::max(nsteps, 0)};
+  size_t total = 0;
+  for (int a = 0; a < 6; ++a) {
+    if (!to[a]) len[a] = 0;
+    total += len[a];
+  }
+  if (!on_device && stage_ready(ctx, total)) {
+    StageCopy C;
+    size_t at[7] = {0};
+    for (int a = 0; a < 6; ++a) {
+      at[a + 1] = at[a] + len[a] * D;
+      if (len[a] == 0) continue;
+      C.from[C.count] = from[a];
+      C.to[C.count] = reinterpret_cast<double*>(ctx->stage.dev + at[a]);
+      C.n[C.count++] = len[a];
+    }
+    int rc = stage_launch(ctx, C);
+    if (rc) return rc;
+    TC_CUDA_TRY(cudaStreamSynchronize(s));
+    for (int a = 0; a < 6; ++a)
+      if (len[a]) memcpy(to[a], ctx->stage.host + at[a], len[a] * D);
+    return TC_OK;
+  }
+  for (int a = 0; a < 6; ++a)
+    if (len[a]) TC_CUDA_TRY(cudaMemcpyAsync(to[a], from[a], len[a] * D, kind, s));
+  if (!on_device) TC_CUDA_TRY(cudaStreamSynchronize(s));
+  return TC_OK;
+}
+
+}  // namespace
+
 extern "C" int tc_rk4_store(tc_ctx* ctx, double* xA, double* zetaA, double* xV, double* xQ,
                             double* kineticEnergy, int on_device) {
   int rc = begin(ctx);
@@ -546,17 +668,7 @@ extern "C" int tc_rk4_store(tc_ctx* ctx, double* xA, double* zetaA, double* xV, 
     tc_record_error("tc_rk4_store: no RK4 state loaded");
     return TC_ERR_STATE;
   }
-  cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-  const size_t D = sizeof(double);
-  cudaStream_t s = ctx->stream;
-  if (xA && R.nA) TC_CUDA_TRY(cudaMemcpyAsync(xA, R.x0A.ptr, 3 * (size_t)R.nA * D, kind, s));
-  if (zetaA && R.nA) TC_CUDA_TRY(cudaMemcpyAsync(zetaA, R.z0.ptr, (size_t)R.nA * D, kind, s));
-  if (xV && R.nV) TC_CUDA_TRY(cudaMemcpyAsync(xV, R.x0V.ptr, 3 * (size_t)R.nV * D, kind, s));
-  if (xQ && R.nQ) TC_CUDA_TRY(cudaMemcpyAsync(xQ, R.x0Q.ptr, 3 * (size_t)R.nQ * D, kind, s));
-  if (kineticEnergy && R.nA)
-    TC_CUDA_TRY(cudaMemcpyAsync(kineticEnergy, R.ke.ptr, (size_t)R.nA * D, kind, s));
-  if (!on_device) TC_CUDA_TRY(cudaStreamSynchronize(s));
-  return TC_OK;
+  return rk4_store(ctx, xA, zetaA, xV, xQ, kineticEnergy, nullptr, 0, on_device);
 }
 
 // One RK4 stage over the given target ranges: the pair sums of all three
@@ -885,22 +997,30 @@ int rk4_advance_enqueue(tc_ctx* ctx, double dt, int nsteps) {
   return TC_OK;
 }
 
-// After the steps of a host-array call: queues the device scans of the new
-// positions and (when the caller wants it) vorticity, the read-back of
-// totalKE and the state (tc_rk4_store, which synchronises). The caller then
-// reads the scans' outcome with scan_results_status(ctx, out, 2).
+// After the steps of a host-array call: totalKE and the state go back to the host, and
+// the new positions and (when the caller wants it) vorticity are scanned for NaN/Inf:
+// small results on the host, which holds them, others on the device. *status is
+// what the scan found, for the caller to return when it is done.
 int rk4_results_to_host(tc_ctx* ctx, double* xA, double* zetaA, double* xV, double* xQ,
-                        int nsteps, double* totalKE, double* kineticEnergy, HostArray out[2]) {
+                        int nsteps, double* totalKE, double* kineticEnergy, int* status) {
   tcb::Rk4State& R = ctx->rk;
-  out[0] = HostArray{R.x0A.as<double>(), 3 * (size_t)R.nA, "xA (result)"};
-  out[1] = HostArray{zetaA ? R.z0.as<double>() : nullptr, (size_t)R.nA,
-                     R.strat ? "relVortA (result)" : "zetaA (result)"};
+  const char* const zname = R.strat ? "relVortA (result)" : "zetaA (result)";
+  const size_t n = (size_t)R.nA;
+  *status = TC_OK;
+  if (4 * n * sizeof(double) <= tcb::HostStage::kStageBytes && (xA || n == 0)) {
+    const int rc = rk4_store(ctx, xA, zetaA, xV, xQ, kineticEnergy, totalKE, nsteps, 0);
+    if (rc) return rc;
+    const HostArray out[2] = {{xA, 3 * n, "xA (result)"}, {zetaA, n, zname}};
+    *status = check_finite_host_all(out, 2);
+    return TC_OK;
+  }
+  const HostArray out[2] = {{R.x0A.as<double>(), 3 * n, "xA (result)"},
+                            {zetaA ? R.z0.as<double>() : nullptr, n, zname}};
   int rc = scan_results_device(ctx, out, 2);
   if (rc) return rc;
-  if (totalKE && nsteps > 0)
-    TC_CUDA_TRY(cudaMemcpyAsync(totalKE, R.totalKE.ptr, (size_t)nsteps * sizeof(double),
-                                cudaMemcpyDeviceToHost, ctx->stream));
-  return tc_rk4_store(ctx, xA, zetaA, xV, xQ, kineticEnergy, 0);
+  if ((rc = rk4_store(ctx, xA, zetaA, xV, xQ, kineticEnergy, totalKE, nsteps, 0))) return rc;
+  *status = scan_results_status(ctx, out, 2);
+  return TC_OK;
 }
 
 // Error return of a host-array call whose work is queued: waits for it, so
@@ -936,10 +1056,10 @@ extern "C" int tc_rk4_step(tc_ctx* ctx, double* xA, double* zetaA, const double*
   if ((rc = rk4_advance_enqueue(ctx, dt, nsteps))) return fail_queued(ctx, rc, false);
   if ((rc = rk4_host_inputs(xA, zetaA, areaA, nA, xV, nV, xQ, nQ)))
     return fail_queued(ctx, rc, true);
-  HostArray out[2];
-  if ((rc = rk4_results_to_host(ctx, xA, zetaA, xV, xQ, nsteps, totalKE, kineticEnergy, out)))
+  int status;
+  if ((rc = rk4_results_to_host(ctx, xA, zetaA, xV, xQ, nsteps, totalKE, kineticEnergy, &status)))
     return rc;
-  return scan_results_status(ctx, out, 2);
+  return status;
 }
 
 extern "C" int tc_rk4_step_device(tc_ctx* ctx, double* xA, double* zetaA, const double* areaA,
@@ -988,8 +1108,8 @@ extern "C" int tc_strat_rk4_step(tc_ctx* ctx, double* xA, const double* absVortA
   if ((rc = check_finite_host_all(in, 2)) ||
       (rc = rk4_host_inputs(xA, absVortA, areaA, nA, xV, nV, xQ, nQ)))
     return fail_queued(ctx, rc, true);
-  HostArray out[2];
-  if ((rc = rk4_results_to_host(ctx, xA, relVortA, xV, xQ, nsteps, totalKE, kineticEnergy, out)))
+  int status;
+  if ((rc = rk4_results_to_host(ctx, xA, relVortA, xV, xQ, nsteps, totalKE, kineticEnergy, &status)))
     return rc;
   if (relVortV && nV) {
     tcb::DevBuf rv;
@@ -1000,7 +1120,7 @@ extern "C" int tc_strat_rk4_step(tc_ctx* ctx, double* xA, const double* absVortA
     TC_CUDA_TRY(cudaMemcpyAsync(relVortV, rv.ptr, nV * D, cudaMemcpyDeviceToHost, ctx->stream));
     TC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   }
-  return scan_results_status(ctx, out, 2);
+  return status;
 }
 
 // Pair-kernel variants (the launch shapes the autotuner searches).
@@ -1114,6 +1234,7 @@ extern "C" int tc_reset_rk4(tc_ctx* ctx) {
   for (DevBuf* b : bufs) b->release();
   ctx->partial.release();
   tc_advance_graph_free(ctx);
+  tc_adjoint_free(ctx);
   R.ready = false;
   R.ordered = false;
   R.nA = R.nV = R.nQ = 0;

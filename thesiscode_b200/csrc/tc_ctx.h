@@ -79,6 +79,21 @@ struct SegDesc {
   long long perm_len;  // entries in perm
 };
 
+// Host arrays of small calls go through one page-locked buffer, which the GPU reads or
+// writes itself, in one kernel each way: five copies from and to pageable memory, each
+// queued or waited for by itself, take longer than a small step (a BVERK4 call on a
+// level-2 grid: 163 us with them, 81 without; the level-5 Voronoi step 679 and 589).
+// Owned by the context, kStageBytes, which the driver hands out of a larger page-locked
+// block in microseconds; larger calls copy array by array.
+struct HostStage {
+  static constexpr size_t kStageBytes = size_t(512) << 10;
+  char* host = nullptr;
+  char* dev = nullptr;         // the same memory, as the GPU sees it
+  cudaEvent_t read = nullptr;  // the last kernel that reads or writes the buffer
+  ~HostStage() { release(); }
+  void release();
+};
+
 // RK4 state and scratch kept on the device between calls (the reference's
 // activePanelsInput/Stage1..4/newActivePanelsX family, :34-71, laid out for
 // the fused stage epilogue: only the running sum of the stages is kept).
@@ -110,6 +125,8 @@ struct tc_batch_plan;            // batched-ensemble plan (batch.cu)
 struct tc_advance_graph;         // captured RK4 steps of tc_rk4_advance (api.cu)
 void tc_advance_graph_free(tc_ctx* ctx);
 void tc_batch_free(tc_ctx* ctx);
+struct tc_adjoint_work;          // buffers of the adjoint (adjoint.cu)
+void tc_adjoint_free(tc_ctx* ctx);
 
 struct tc_ctx {
   int device = 0;
@@ -135,6 +152,7 @@ struct tc_ctx {
   tcb::DevBuf partial;    // pair-kernel partial sums
   tcb::DevBuf scratch[6]; // one-call buffers (velocity entry points)
   tcb::DevBuf grid_buf[6];  // tc_icos_grid_device: edge and panel tables, prefix sums
+  tcb::HostStage stage;     // host arrays of small calls
   tcb::DevBuf check_buf;    // first non-finite index of each result array scanned on the device
   tcb::Rk4State rk;
   // instrumentation (tc_stats): kernels launched, and CUDA-event time of the
@@ -147,6 +165,7 @@ struct tc_ctx {
   double pair_ms = 0.0;
   tc_batch_plan* batch = nullptr;
   tc_advance_graph* agraph = nullptr;
+  tc_adjoint_work* adjoint = nullptr;
   int rk4_graphs = 1;  // tc_rk4_advance graph replay: 0 never, 1 small problems, 2 always
   // checked build: the device's violation record, and per-site caps on the declared
   // extents (tc_bounds_cap)
