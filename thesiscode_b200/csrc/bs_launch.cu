@@ -235,26 +235,30 @@ static int count_tiles(const SegDesc* segs, int nseg, int tb) {
 // Chunk length of any launch. CTAs cost unequal times (near or far tiles, frame or
 // wide form), so a launch ends with a tail of about one CTA's length: chunks are cut
 // for kWaves waves, as far as they keep min_len sources (the prologue's share) and
-// their number kMostChunks (the epilogue's). FP32C level 6 refined in 4 / 8 / 24 / 48
-// chunks: 5.30 / 5.16 / 5.06 / 5.04 ms, level 7 in 1 / 4 / 16 / 24: 44.0 / 41.6 / 41.0 /
-// 40.8; FP64 level 5 in 8 / 24 / 48: 0.604 / 0.474 / 0.436 ms. Launches that stay below
-// three waves that way fill whole waves instead (choose_chunks), or, with the shapes
-// for few sources, minimise the model's time.
+// their number stays within `most` (the epilogue's). FP32C level 6 refined in 4 / 8 / 24
+// / 48 chunks: 5.30 / 5.16 / 5.06 / 5.04 ms, level 7 in 1 / 4 / 16 / 24: 44.0 / 41.6 /
+// 41.0 / 40.8, level 5 panels alone in 10 / 20 / 40: 0.178 / 0.161 / 0.150; FP64 level 5
+// in 8 / 24 / 48: 0.604 / 0.474 / 0.436 ms, its panels alone in 10 / 16 / 64: 0.342 /
+// 0.313 / 0.303. Launches that stay below one wave that way minimise a model's time or
+// fill the wave (choose_chunks). With the shapes for few sources an epilogue costs as much
+// as finer chunks gain (ten level-4 FP64 steps 2.03 ms by the model, 2.10 in 53 chunks):
+// they take the model below three waves.
 constexpr int kWaves = 32;
 
 static int chunk_length(const tc_ctx* ctx, const PairCfg& cfg, int slots, int tiles, int n,
                         int max_chunks) {
   const bool fp64 = ctx->precision == TC_FP64;
-  const int min_len = fp64 ? 448 : 768, most = std::min(max_chunks, fp64 ? 48 : 24);
+  const int gran = fp64 && ctx->var64 >= kAuto64Small ? 16 : cfg.ts;
+  const bool few = fp64 ? ctx->var64 == kAuto64Small : ctx->var32 == kAutoFewVariant;
+  const int min_len = fp64 ? (few ? 448 : 256) : (few ? 768 : 512);
+  const int most = std::min(max_chunks, fp64 ? (few ? 48 : 64) : (few ? 24 : 40));
   const long long S = std::min<long long>(
       {((long long)kWaves * slots + tiles - 1) / tiles, n / min_len, (long long)most});
-  const int gran = fp64 && ctx->var64 >= kAuto64Small ? 16 : cfg.ts;
-  if (S * tiles >= 3LL * slots) {
+  if (S * tiles >= (few ? 3LL : 1LL) * slots) {
     const int len = std::max(gran, (int)(n / S) / gran * gran);  // one chunk more, if there is room
     return (n + len - 1) / len <= max_chunks ? len : len + gran;
   }
-  const bool few = fp64 ? ctx->auto64 : ctx->auto32 && ctx->var32 == kAutoFewVariant;
-  if (few)
+  if (fp64 ? ctx->auto64 : ctx->auto32 && few)
     return fine_chunk_len(tiles, n, ctx->num_sms, slots, cfg.nt / 32, fp64 ? 12 : 16, max_chunks,
                           gran);
   return whole_chunk_len(tiles, n, cfg.ts, slots, ctx->min_chunk, max_chunks);
