@@ -331,31 +331,54 @@ __device__ __forceinline__ void adj_row_source(const double4 q, const double4 w,
                                                const double* g0, const double* g1, const double* g2,
                                                const double* v0, const double* v1, const double* v2,
                                                double (*a)[kRowSums]) {
+  // operation by operation over the rows, so that a source's register is read for all of
+  // them at once (level 6: 10.36 ms a product row by row, 10.23 so)
+  double D[TPT], r[TPT], c[TPT];
 #pragma unroll
-  for (int t = 0; t < TPT; ++t) {
-    double D = fma(-q.x, x0[t], one_plus_d2);
-    D = fma(-q.y, x1[t], D);
-    D = fma(-q.z, x2[t], D);
-    double r = adj_rcp_n<NEWTON>(D);
-    if (MASK) r = (k == row[t]) ? 0.0 : r;  // zero-padded sources give r * 0 anyway
-    // (G_j x_j).v_i + (G_i x_i).v_j
-    double c = q.w * v0[t];
-    c = fma(w.x, v1[t], c);
-    c = fma(w.y, v2[t], c);
-    c = fma(g0[t], w.z, c);
-    c = fma(g1[t], w.w, c);
-    c = fma(g2[t], vz, c);
-    const double cr2 = c * (r * r);
-    a[t][0] = fma(r, q.w, a[t][0]);
-    a[t][1] = fma(r, w.x, a[t][1]);
-    a[t][2] = fma(r, w.y, a[t][2]);
-    a[t][3] = fma(cr2, q.x, a[t][3]);
-    a[t][4] = fma(cr2, q.y, a[t][4]);
-    a[t][5] = fma(cr2, q.z, a[t][5]);
-    a[t][6] = fma(r, w.z, a[t][6]);
-    a[t][7] = fma(r, w.w, a[t][7]);
-    a[t][8] = fma(r, vz, a[t][8]);
+  for (int t = 0; t < TPT; ++t) D[t] = fma(-q.x, x0[t], one_plus_d2);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) D[t] = fma(-q.y, x1[t], D[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) D[t] = fma(-q.z, x2[t], D[t]);
+  // (G_j x_j).v_i + (G_i x_i).v_j
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = q.w * v0[t];
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = fma(w.x, v1[t], c[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = fma(w.y, v2[t], c[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = fma(g0[t], w.z, c[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = fma(g1[t], w.w, c[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = fma(g2[t], vz, c[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) r[t] = adj_rcp_n<NEWTON>(D[t]);
+  if (MASK) {  // zero-padded sources give r * 0 anyway
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) r[t] = (k == row[t]) ? 0.0 : r[t];
   }
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) c[t] = c[t] * (r[t] * r[t]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][0] = fma(r[t], q.w, a[t][0]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][1] = fma(r[t], w.x, a[t][1]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][2] = fma(r[t], w.y, a[t][2]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][6] = fma(r[t], w.z, a[t][6]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][7] = fma(r[t], w.w, a[t][7]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][8] = fma(r[t], vz, a[t][8]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][3] = fma(c[t], q.x, a[t][3]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][4] = fma(c[t], q.y, a[t][4]);
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) a[t][5] = fma(c[t], q.z, a[t][5]);
 }
 
 template <int TPT, int NEWTON, int UNROLL>
