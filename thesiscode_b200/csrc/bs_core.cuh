@@ -493,9 +493,12 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P)
 //   origin. With a = -c.s_k and b = -c.t_i (minus the offsets' third coordinates,
 //   as e3 = c), the identity 1 - x_i.x_k = a + b - a b - s_x t_x - s_y t_y holds
 //   on and off the sphere for a unit origin c, so
-//       D/2 = a_k (1 - b_i) + (b_i + delta^2) - s_k,x t_i,x - s_k,y t_i,y
-//   takes 3 FMA with the targets' values in registers, a, b and b + delta^2 from
-//   FP64; and T' += r (G_k x'_k), x'_k = R x_k = (s_x, s_y, 1 - a) (G x' from FP64,
+//       (D/2) / (1 - b_i) = a_k + [(b_i + delta^2) - s_k,x t_i,x - s_k,y t_i,y] / (1 - b_i)
+//   takes an addition and 2 FMA with the targets' values, divided by 1 - b_i in
+//   FP64, in registers. (Multiplying a_k by 1 - b_i rounded to FP32 would shift
+//   all of a target's far terms by the same 2^-25: level 8, 24,575 rows, rms error
+//   1.32e-8 where the four products gave 1.12e-8.) T' += r (G_k x'_k) is then 1 - b_i times the sum, taken
+//   out at the end, near sums being scaled up to it; x'_k = R x_k = (s_x, s_y, 1 - a) (G x' from FP64,
 //   one rounding). In the rotated frame the first two coordinates of x'_k are
 //   small tangential offsets and the third is about 1, so the large common part
 //   of the sum (about sum r G) sits in the third coordinate only, and u_i = x_i x
@@ -581,6 +584,7 @@ struct SpSmem {
   double frame[12];        // e1, e2, e3 (rows), origin c
   double csum[3][NT / 32]; // per-warp sums of the target positions
   double acc[SMACC ? 3 * T * NT : 1];  // FP64 accumulators [c][t][thread] (SMACC)
+  double om[T * NT];                   // 1 - b of the targets [t][thread]
   float4 lo[HILO ? TS / 2 : 1];        // HILO: low parts (slx_k, slx_k+1, sly_k, sly_k+1)
   float2 loz[HILO ? TS / 2 : 1];       // HILO: low parts of (a_k, a_k+1)
   float tlo[HILO ? 3 * T * NT : 1];    // HILO: low parts of (-t_x, -t_y, -b) [c][t][thread]
@@ -600,18 +604,18 @@ __device__ __forceinline__ float2 rcp2(float2 D) {
 // without, 41.2 with. Errors against FP64 are the same to two digits.
 template <int T, bool SHARE>
 __device__ __forceinline__ void sp_far_step(const float4 a, const float4 b, const float4 c,
-                                            const float2* ntx, const float2* nty, const float2* omb,
-                                            const float2* bd, float2* fx, float2* fy, float2* fz) {
+                                            const float2* ftx, const float2* fty, const float2* bd,
+                                            float2* fx, float2* fy, float2* fz) {
   const float2 sx = make_float2(a.x, a.y), sy = make_float2(a.z, a.w);
   const float2 ak = make_float2(b.x, b.y), gx = make_float2(b.z, b.w);
   const float2 gy = make_float2(c.x, c.y), gz = make_float2(c.z, c.w);
   float2 D[T];
 #pragma unroll
-  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(ak, omb[t], bd[t]);
+  for (int t = 0; t < T; ++t) D[t] = __fadd2_rn(ak, bd[t]);
 #pragma unroll
-  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sx, ntx[t], D[t]);
+  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sx, ftx[t], D[t]);
 #pragma unroll
-  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sy, nty[t], D[t]);
+  for (int t = 0; t < T; ++t) D[t] = __ffma2_rn(sy, fty[t], D[t]);
   if (SHARE && T >= 2) {
     const float2 r = rcp2(__fmul2_rn(D[0], D[1]));
     const float2 r0 = __fmul2_rn(r, D[1]);
@@ -715,15 +719,14 @@ __device__ __forceinline__ void sp_stage(const double4* __restrict__ src, int ts
 
 // Far source pairs [j0, j1) of the staged tile against the thread's targets.
 template <int T, int UNROLL, bool SHARE, class Smem>
-__device__ __forceinline__ void sp_far_run(const Smem& sm, int j0, int j1, const float2 (&ntx)[T],
-                                           const float2 (&nty)[T], const float2 (&omb)[T],
-                                           const float2 (&bd)[T], float2 (&fx)[T], float2 (&fy)[T],
-                                           float2 (&fz)[T]) {
+__device__ __forceinline__ void sp_far_run(const Smem& sm, int j0, int j1, const float2 (&ftx)[T],
+                                           const float2 (&fty)[T], const float2 (&bd)[T],
+                                           float2 (&fx)[T], float2 (&fy)[T], float2 (&fz)[T]) {
   static_assert(UNROLL % 2 == 0, "an even number of source pairs per loop body");
 #pragma unroll UNROLL / 2
   for (int j = j0; j < j1; j += 2) {
-    sp_far_step<T, SHARE>(sm.a[j], sm.b[j], sm.c[j], ntx, nty, omb, bd, fx, fy, fz);
-    sp_far_step<T, false>(sm.a[j + 1], sm.b[j + 1], sm.c[j + 1], ntx, nty, omb, bd, fx, fy, fz);
+    sp_far_step<T, SHARE>(sm.a[j], sm.b[j], sm.c[j], ftx, fty, bd, fx, fy, fz);
+    sp_far_step<T, false>(sm.a[j + 1], sm.b[j + 1], sm.c[j + 1], ftx, fty, bd, fx, fy, fz);
   }
 }
 
@@ -735,10 +738,11 @@ __device__ __forceinline__ void sp_far_run(const Smem& sm, int j0, int j1, const
 // otherwise one far test for the whole tile.
 template <int NT, int T, int TS, int FLUSH, int UNROLL, bool SMACC, bool HILO, int FARK, bool SHARE,
           class Smem>
-__device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
-                                       const float2 (&nty)[T], const float2 (&omb)[T],
-                                       const float2 (&bd)[T], const float (&nb)[T],
-                                       const float (&ei)[T], float2 (&fx)[T], float2 (&fy)[T], float2 (&fz)[T],
+__device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ftx)[T],
+                                       const float2 (&fty)[T], const float2 (&bd)[T],
+                                       const float (&ntx)[T], const float (&nty)[T],
+                                       const float (&nb)[T], const float (&ei)[T],
+                                       float2 (&fx)[T], float2 (&fy)[T], float2 (&fz)[T],
                                        SpAcc<NT, T, SMACC>& acc) {
   constexpr int NP = TS / 2;
   constexpr int FP = FLUSH / 2;
@@ -748,7 +752,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
   const bool tile_far = combine_min<NT / 32>(sm.tmin) > lim;
   if (tile_far) {
     for (int jf = 0; jf < NP; jf += FPF) {
-      sp_far_run<T, UNROLL, SHARE>(sm, jf, jf + FPF, ntx, nty, omb, bd, fx, fy, fz);
+      sp_far_run<T, UNROLL, SHARE>(sm, jf, jf + FPF, ftx, fty, bd, fx, fy, fz);
 #pragma unroll
       for (int t = 0; t < T; ++t) {
         acc.add(0, t, (double)__fadd_rn(fx[t].x, fx[t].y));
@@ -762,7 +766,7 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
   for (int jf = 0; jf < NP; jf += FP) {
     const bool far = PERSEG && __uint_as_float(sm.tmin[jf / FP]) > lim;
     if (far) {
-      sp_far_run<T, UNROLL, SHARE>(sm, jf, jf + FP, ntx, nty, omb, bd, fx, fy, fz);
+      sp_far_run<T, UNROLL, SHARE>(sm, jf, jf + FP, ftx, fty, bd, fx, fy, fz);
     } else {
       // HILO: d = (s_hi - t_hi) + (s_lo - t_lo), accurate to a few ulps of d itself
       float ntl[HILO ? 3 * T : 1];
@@ -786,8 +790,8 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
         }
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-          float2 dx = __fadd2_rn(sx, ntx[t]);
-          float2 dy = __fadd2_rn(sy, nty[t]);
+          float2 dx = __fadd2_rn(sx, make_float2(ntx[t], ntx[t]));
+          float2 dy = __fadd2_rn(sy, make_float2(nty[t], nty[t]));
           float2 dz = __fadd2_rn(ak, make_float2(nb[t], nb[t]));  // -(s_z - t_z)
           if (HILO) {
             dx = __fadd2_rn(dx, __fadd2_rn(make_float2(lo.x, lo.y), make_float2(ntl[t], ntl[t])));
@@ -805,12 +809,13 @@ __device__ __forceinline__ void sp_sum(const Smem& sm, const float2 (&ntx)[T],
         }
       }
     }
-    const float zsign = far ? 1.f : -1.f;
 #pragma unroll
     for (int t = 0; t < T; ++t) {
-      acc.add(0, t, (double)__fadd_rn(fx[t].x, fx[t].y));
-      acc.add(1, t, (double)__fadd_rn(fy[t].x, fy[t].y));
-      acc.add(2, t, (double)(zsign * __fadd_rn(fz[t].x, fz[t].y)));
+      // near: scaled up to the far sums, and z was summed with the other sign
+      const double up = far ? 1.0 : sm.om[t * NT + threadIdx.x];
+      acc.add(0, t, up * (double)__fadd_rn(fx[t].x, fx[t].y));
+      acc.add(1, t, up * (double)__fadd_rn(fy[t].x, fy[t].y));
+      acc.add(2, t, (far ? up : -up) * (double)__fadd_rn(fz[t].x, fz[t].y));
       fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
     }
   }
@@ -901,8 +906,8 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
   const double* fr = sm.frame;
   const double cx = fr[9], cy = fr[10], cz = fr[11];
 
-  float2 ntx[T], nty[T], omb[T], bd[T];  // -t_x, -t_y, 1 - b, b + delta^2
-  float nb[T], ei[T];  // near form only, paired on use: -b, e
+  float2 ftx[T], fty[T], bd[T];  // far: (-t_x, -t_y, b + delta^2) / (1 - b)
+  float ntx[T], nty[T], nb[T], ei[T];  // near, paired on use: -t_x, -t_y, -b, e
   float2 fx[T], fy[T], fz[T];
   SpAcc<NT, T, SMACC> acc;
   acc.init(sm.acc);
@@ -931,14 +936,22 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
       sm.tlo[(2 * T + t) * NT + threadIdx.x] = -(float)(bid - (double)b);
     }
     const double E = (1.0 - (px * px + py * py + pz * pz)) + 2.0 * d2;
-    const float om = (float)(1.0 - bid), bdf = (float)(bid + d2);
-    ntx[t] = make_float2(-tx, -tx);
-    nty[t] = make_float2(-ty, -ty);
-    omb[t] = make_float2(om, om);
-    bd[t] = make_float2(bdf, bdf);
+    rho2 = fmaxf(rho2, norm2_f32(tx, ty, b));
+    double om = 1.0 - bid;
+    if (!(om > 0.5)) {  // more than 60 degrees from the origin: no tile of this CTA is far
+      om = 1.0;
+      rho2 = __int_as_float(0x7f800000);
+    }
+    const double sc = rcp_f64(om);
+    const float fx0 = (float)(-txd * sc), fy0 = (float)(-tyd * sc), b0 = (float)((bid + d2) * sc);
+    ftx[t] = make_float2(fx0, fx0);
+    fty[t] = make_float2(fy0, fy0);
+    bd[t] = make_float2(b0, b0);
+    sm.om[t * NT + threadIdx.x] = om;
+    ntx[t] = -tx;
+    nty[t] = -ty;
     nb[t] = -b;
     ei[t] = (float)E + kSelfBias;
-    rho2 = fmaxf(rho2, norm2_f32(tx, ty, b));
     fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
   }
   warp_store_max(rho2, sm.rho);
@@ -946,16 +959,17 @@ __device__ __forceinline__ void fp32c_sp_unit(const double* __restrict__ x, cons
     __syncthreads();
     sp_stage<NT, TS, HILO>(src, ts, c1, fr, sm, ub);
     __syncthreads();
-    sp_sum<NT, T, TS, FLUSH, UNROLL, SMACC, HILO, FARK, SHARE>(sm, ntx, nty, omb, bd, nb, ei, fx,
-                                                               fy, fz, acc);
+    sp_sum<NT, T, TS, FLUSH, UNROLL, SMACC, HILO, FARK, SHARE>(
+        sm, ftx, fty, bd, ntx, nty, nb, ei, fx, fy, fz, acc);
   }
   // back to the global frame: T = R^T T'
 #pragma unroll
   for (int t = 0; t < T; ++t) {
     const int pos = tile0 + (int)threadIdx.x + t * NT;
     if (pos < i_end) {
-      double ax = acc.get(0, t);
-      const double ay = acc.get(1, t), az = acc.get(2, t);
+      const double sc = rcp_f64(sm.om[t * NT + threadIdx.x]);
+      double ax = acc.get(0, t) * sc;
+      const double ay = acc.get(1, t) * sc, az = acc.get(2, t) * sc;
       if (SHARE && ((bad >> t) & 1u)) ax = __longlong_as_double(0x7ff8000000000000ll);
       if (TC_BC(ub.rec, BC_PAIR_OUT, ub.out_base + pos, ub.out_len))
         out[pos] = fma(fr[0], ax, fma(fr[3], ay, fr[6] * az));

@@ -17,10 +17,10 @@ namespace {
 constexpr int kChains = 8;
 
 // The far-form pair step of the FP32C kernel itself (tcb::sp_far_run: per
-// source pair and three targets 18 FFMA2 and six MUFU reciprocals, or 21 and four
-// in every second source pair, which comes from shared memory) with the default variant's shape:
-// 128 threads, 3 targets per thread, 4 CTAs per SM, 4 source pairs per
-// unrolled body. The 128 source pairs stay resident in shared memory. There
+// source pair and three targets 3 FADD2, 15 FFMA2 and six MUFU reciprocals, or 3
+// FMUL2 more and four in every second source pair, which comes from shared memory)
+// with the default variant's shape: 128 threads, 3 targets per thread, 4 CTAs per SM,
+// 4 source pairs per unrolled body. The 128 source pairs stay resident in shared memory. There
 // is no staging, no far test, no flush and no near tile, so its rate
 // (pairs/s, one pair = one target x one source) is the ceiling of the pair
 // loop's instruction mix on this GPU.
@@ -42,18 +42,17 @@ __global__ void __launch_bounds__(kFarNT, kFarMinB) probe_far_pairs(int iters, f
     tile.c[j] = make_float4(s, -s, s, 2.0f * s);                      // G y', G z'
   }
   __syncthreads();
-  float2 ntx[kFarT], nty[kFarT], omb[kFarT], bd[kFarT], fx[kFarT], fy[kFarT], fz[kFarT];
+  float2 ntx[kFarT], nty[kFarT], bd[kFarT], fx[kFarT], fy[kFarT], fz[kFarT];
 #pragma unroll
   for (int t = 0; t < kFarT; ++t) {
     const float u = 1e-4f * (float)(threadIdx.x + 32 * t);
     ntx[t] = make_float2(-u, -u);
     nty[t] = make_float2(u, u);
-    omb[t] = make_float2(1.0f - 0.5f * u, 1.0f - 0.5f * u);
     bd[t] = make_float2(0.5f + u, 0.5f + u);
     fx[t] = fy[t] = fz[t] = make_float2(0.f, 0.f);
   }
   for (int i = 0; i < iters; ++i)
-    tcb::sp_far_run<kFarT, 4, true>(tile, 0, kFarNP, ntx, nty, omb, bd, fx, fy, fz);
+    tcb::sp_far_run<kFarT, 4, true>(tile, 0, kFarNP, ntx, nty, bd, fx, fy, fz);
   float s = 0.f;
 #pragma unroll
   for (int t = 0; t < kFarT; ++t) s += fx[t].x + fx[t].y + fy[t].x + fy[t].y + fz[t].x + fz[t].y;
