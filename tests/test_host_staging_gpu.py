@@ -1,7 +1,7 @@
 """Host-array calls through the page-locked staging buffer equal the device-array calls.
 
-A call whose arrays take at most 512 KiB goes through one buffer, a larger one copies array by
-array: the same steps on arrays around that limit, from and to host memory and device memory,
+A call whose arrays take at most 512 KiB goes through one buffer once the context has made 16
+such transfers, before that and where it is larger it copies array by array: the same steps on arrays around that limit, from and to host memory and device memory,
 bit for bit. The buffer is reused: a second load before the first state is stored, and calls
 of other sizes, leave nothing of the first behind."""
 import ctypes
@@ -43,12 +43,33 @@ def device_step(ctx, s, steps):
     return [dev[0].cpu().numpy(), dev[1].cpu().numpy(), dev[3].cpu().numpy(), dev[4].cpu().numpy(), tke, ke.cpu().numpy()]
 
 
+def staging_context(prec, transfers=16):
+    """A context after `transfers` small transfers; by then it has taken (or is about to take) the buffer."""
+    ctx = Context(0, prec)
+    s = state(3, 1, 0, 9)
+    for _ in range(transfers):
+        ctx.rk4_load(*s)
+    return ctx
+
+
+def test_the_buffer_is_taken_between_load_and_store(gpu):
+    """Loads and stores on either side of the transfer from which on the buffer is used."""
+    for transfers in (0, 13, 14, 15, 16, 17):
+        ctx = staging_context("fp64", transfers)
+        for seed in (1, 2):
+            s = state(300, 100, 7, seed)
+            ctx.rk4_load(*s)
+            for a, b in zip(ctx.rk4_store(300, 100, 7), (s[0], s[1], s[3], s[4])):
+                np.testing.assert_array_equal(a, b)
+        ctx.close()
+
+
 # doubles staged on the way in: 5 nA + 3 nV + 3 nQ, at most 65,536
 @pytest.mark.parametrize("prec", ["fp64", "fp32c"])
 @pytest.mark.parametrize("nA,nV,nQ", [(1, 0, 0), (257, 0, 3), (40, 1000, 0), (13107, 0, 0), (13106, 2, 0), (13106, 3, 0),
                                       (9000, 4000, 2845), (9000, 4000, 2846)])
 def test_host_and_device_arrays_agree(gpu, prec, nA, nV, nQ):
-    ctx = Context(0, prec)
+    ctx = staging_context(prec)
     ctx.set_deltas(0.05, 0.05, 0.05)
     for seed, steps in ((1, 1), (2, 3)):
         s = state(nA, nV, nQ, seed)
@@ -58,7 +79,7 @@ def test_host_and_device_arrays_agree(gpu, prec, nA, nV, nQ):
 
 
 def test_a_second_load_replaces_the_first(gpu):
-    ctx = Context(0, "fp64")
+    ctx = staging_context("fp64")
     first, second = state(300, 100, 7, 3), state(200, 50, 0, 4)
     ctx.rk4_load(*first)
     ctx.rk4_load(*second)
@@ -74,7 +95,7 @@ def test_a_second_load_replaces_the_first(gpu):
 
 def test_a_non_finite_result_is_reported_with_its_index(gpu):
     """Finite inputs whose step overflows: the result comes back, and the call says where."""
-    ctx = Context(0, "fp64")
+    ctx = staging_context("fp64")
     xA, z, a, xV, xQ = state(50, 0, 0, 5)
     z[:] = 1e300
     a[:] = 1e300

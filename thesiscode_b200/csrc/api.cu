@@ -122,6 +122,10 @@ bool stage_ready(tc_ctx* ctx, size_t total) {
   }
   tcb::HostStage& S = ctx->stage;
   if (!S.host) {
+    if (S.plain < tcb::HostStage::kPlainFirst) {
+      ++S.plain;
+      return false;
+    }
     void *h = nullptr, *d = nullptr;
     if (cudaHostAlloc(&h, tcb::HostStage::kStageBytes, cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess ||

@@ -83,10 +83,16 @@ struct SegDesc {
 // writes itself, in one kernel each way: five copies from and to pageable memory, each
 // queued or waited for by itself, take longer than a small step (a BVERK4 call on a
 // level-2 grid: 163 us with them, 81 without; the level-5 Voronoi step 679 and 589).
-// Owned by the context, kStageBytes, which the driver hands out of a larger page-locked
-// block in microseconds; larger calls copy array by array.
+// Owned by the context, kStageBytes; larger calls copy array by array. The driver hands
+// it out of a 2 MB page-locked block, in microseconds where one is open and else in 1.3 to
+// 2 ms (every fourth context, or each one where the last was freed): a context takes it
+// once its small transfers have cost about as much more than staged ones, so that one
+// made for a few calls never pays for it (first step of a new level-4 forced state: 2.9 to
+// 4.7 ms with the buffer taken at once, 2.0 to 2.4 without).
 struct HostStage {
   static constexpr size_t kStageBytes = size_t(512) << 10;
+  static constexpr int kPlainFirst = 16;  // transfers, 40 to 80 us saved by each pair of them
+  int plain = 0;                          // copied array by array so far
   char* host = nullptr;
   char* dev = nullptr;         // the same memory, as the GPU sees it
   cudaEvent_t read = nullptr;  // the last kernel that reads or writes the buffer
