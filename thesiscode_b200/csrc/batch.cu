@@ -9,6 +9,7 @@
 // the actual batch, and caches the choice per batch shape.
 #include <algorithm>
 #include <cub/device/device_radix_sort.cuh>
+#include <cstdint>
 #include <cstring>
 #include <map>
 #include <numeric>
@@ -67,18 +68,20 @@ __global__ void ke_segments_kernel(const double* __restrict__ ke, const double* 
 
 }  // namespace
 
-// Host-side plan of one batch shape.
+// Host-side plan of one batch shape and precision.
 struct tc_batch_plan {
   int count = 0;
   std::vector<int> nA, nV, aOff, vOff;
   int nA_tot = 0, nV_tot = 0;
+  int precision = -1;  // of the variant and its items
   int variant = -1, chunk_len = 0, n_items = 0, slots = 0;
+  bool tuned = false;  // variant and chunk_len are the autotuner's
   DevBuf items, segs0, segs1, counters, row_nchunks, row_inst, off_d, cnt_d, keys, keys2, vals,
       sort_tmp, ke_out, partial;
   cudaGraphExec_t graph = nullptr;
-  int graph_steps = -1;
-  double graph_dt = 0.0;
-  std::vector<void*> graph_ptrs;  // every device buffer the graph touches, at capture time
+  // what the captured steps depend on: dt, steps, the context's parameters and the address
+  // of every device buffer they touch
+  std::vector<uint64_t> graph_key;
   cudaStream_t stream = nullptr;  // used when the context runs on the (uncapturable) NULL stream
   ~tc_batch_plan() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -259,6 +262,22 @@ int enqueue_steps(tc_ctx* ctx, tc_batch_plan& B, double dt, int nsteps) {
   return TC_OK;
 }
 
+// What the steps that enqueue_steps queues depend on besides the data in the buffers.
+std::vector<uint64_t> graph_key(const tc_ctx* ctx, const tc_batch_plan& B, double dt, int nsteps) {
+  const tcb::Rk4State& R = ctx->rk;
+  const double vals[5] = {dt, ctx->omega, ctx->delta[0], ctx->delta[1], ctx->delta[2]};
+  std::vector<uint64_t> k(5);
+  memcpy(k.data(), vals, sizeof(vals));
+  for (int v : {nsteps, ctx->precision, (int)R.ordered, B.variant, B.chunk_len, B.n_items, B.slots})
+    k.push_back((uint64_t)v);
+  for (const DevBuf* b :
+       {&R.x0A, &R.z0, &R.areaA, &R.x0V, &R.xiA, &R.ziA, &R.xiV, &R.newA, &R.newZ, &R.newV, &R.src,
+        &R.ke, &R.keBlocks, &R.permA, &R.permV, &B.items, &B.segs0, &B.segs1, &B.counters,
+        &B.row_nchunks, &B.off_d, &B.cnt_d, &B.ke_out, &B.partial})
+    k.push_back((uint64_t)(uintptr_t)b->ptr);
+  return k;
+}
+
 // Time one stage-0 pair launch of each (variant, chunk) candidate; keep the best.
 // Candidate launch shapes: the default of each precision first, then the
 // shapes that were fastest on some workload of the level-7 sweep, all with the
@@ -338,12 +357,12 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
   tc_batch_plan& B = *ctx->batch;
   const bool same_shape = B.count == count && std::equal(B.nA.begin(), B.nA.end(), nA) &&
                           std::equal(B.nV.begin(), B.nV.end(), nV);
-  if (!same_shape) {
+  if (!same_shape || B.precision != ctx->precision) {
     if (B.graph) cudaGraphExecDestroy(B.graph);
     B.graph = nullptr;
-    B.graph_steps = -1;
     B.variant = -1;
   }
+  B.precision = ctx->precision;
   B.count = count;
   B.nA.assign(nA, nA + count);
   B.nV.assign(nV, nV + count);
@@ -408,14 +427,17 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
   }
   if ((rc = upload_segments(ctx, B))) return rc;
   if ((rc = tc_rk4_pack_sources(ctx))) return rc;
-  if (B.variant < 0) {
-    if (flags & TC_BATCH_AUTOTUNE) {
-      if ((rc = autotune(ctx, B))) return rc;
-    } else {
-      const int v = ctx->precision == TC_FP64 ? (ctx->auto64 ? tcb::kAuto64Default : ctx->var64)
-                                              : ctx->var32;
-      if ((rc = build_items(ctx, B, v, 4096))) return rc;
+  // a plan's launch shape stays until the caller asks for another: for tuning, or by
+  // tc_set_pair_variant
+  const bool fp64 = ctx->precision == TC_FP64, tune = (flags & TC_BATCH_AUTOTUNE) != 0;
+  const bool fixed = !(fp64 ? ctx->auto64 : ctx->auto32);
+  const int plain = fp64 ? (ctx->auto64 ? tcb::kAuto64Default : ctx->var64) : ctx->var32;
+  if (B.variant < 0 || (tune && !B.tuned) || (!tune && fixed && B.variant != plain)) {
+    if ((rc = tune ? autotune(ctx, B) : build_items(ctx, B, plain, 4096))) {
+      B.variant = -1;
+      return rc;
     }
+    B.tuned = tune;
     if ((rc = tc_rk4_pack_sources(ctx))) return rc;  // autotuning ran stage-0 launches only
   }
   // the stage-0 epilogue's per-block kinetic-energy buffer: sized before any capture
@@ -423,14 +445,9 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
                               sizeof(double))))
     return rc;
   if (nsteps > 0) {
-    const std::vector<void*> ptrs = {R.x0A.ptr, R.z0.ptr, R.areaA.ptr, R.x0V.ptr, R.xiA.ptr,
-                                     R.ziA.ptr, R.xiV.ptr, R.newA.ptr, R.newZ.ptr, R.newV.ptr,
-                                     R.src.ptr, R.ke.ptr, R.keBlocks.ptr, R.permA.ptr, R.permV.ptr,
-                                     B.items.ptr, B.segs0.ptr, B.segs1.ptr, B.counters.ptr,
-                                     B.row_nchunks.ptr, B.off_d.ptr, B.cnt_d.ptr, B.ke_out.ptr,
-                                     B.partial.ptr};
     if (flags & TC_BATCH_GRAPH) {
-      if (!B.graph || B.graph_steps != nsteps || B.graph_dt != dt || B.graph_ptrs != ptrs) {
+      const std::vector<uint64_t> key = graph_key(ctx, B, dt, nsteps);
+      if (!B.graph || B.graph_key != key) {
         if (B.graph) cudaGraphExecDestroy(B.graph);
         B.graph = nullptr;
         cudaGraph_t g;
@@ -444,9 +461,7 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
         }
         TC_CUDA_TRY(cudaGraphInstantiate(&B.graph, g, 0));
         cudaGraphDestroy(g);
-        B.graph_steps = nsteps;
-        B.graph_dt = dt;
-        B.graph_ptrs = ptrs;
+        B.graph_key = key;
       }
       TC_CUDA_TRY(cudaGraphLaunch(B.graph, ctx->stream));
     } else if ((rc = enqueue_steps(ctx, B, dt, nsteps))) {
