@@ -222,6 +222,7 @@ int launch_batch_pairs(tc_ctx* ctx, tc_batch_plan& B, int stage) {
   L.src = ctx->rk.src.as<double4>();
   L.partial = B.partial.as<double>();
   L.stride = (size_t)(B.nA_tot + B.nV_tot);
+  L.care = std::min(ctx->delta[0] * ctx->delta[0], ctx->delta[1] * ctx->delta[1]) < tcb::kCareD;
   L.bc = ctx->bc_rec;
   L.n_segs = (int)tcb::bc_extent(ctx, tcb::BC_BATCH_SEG, 2 * B.count);
   L.src_len =

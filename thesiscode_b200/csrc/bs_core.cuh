@@ -50,6 +50,7 @@ struct PairLaunch {
   int chunk_len;        // sources per blockIdx.y chunk (multiple of the tile)
   double* partial;      // partial[(chunk*3 + c)*n_out + row]
   int n_out;
+  bool care;            // FP64: a segment with frames has d2 < kCareD
   BoundsRec* bc;        // checked build: violation record (null: release build)
   long long src_len;    // checked build: packed sources in src
   long long partial_len;  // checked build: doubles in partial
@@ -70,13 +71,19 @@ struct UnitBounds {
 // (measured over [1, 2): 1.1e-16). Two Newton steps would take 4, the
 // compiler's IEEE division about 14.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double rcp_f64(double d) {
+__device__ __forceinline__ double rcp_seed_f64(double d) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  return r;
+}
+
+__device__ __forceinline__ double rcp_refine_f64(double d, double r) {
   double e = fma(-d, r, 1.0);
   e = fma(e, e, e);
   return fma(r, e, r);
 }
+
+__device__ __forceinline__ double rcp_f64(double d) { return rcp_refine_f64(d, rcp_seed_f64(d)); }
 
 __device__ __forceinline__ float rcp_approx_f32(float d) {
   float r;
@@ -141,6 +148,18 @@ __device__ __forceinline__ double frame_dot(const double* e, double vx, double v
 //   u = x_i x T ignores) is taken out in the frame, where x_i is (small, small,
 //   about 1), before T' is rotated back. The denominator keeps an absolute error
 //   of ulps of |s| |t| where 1 - x.y keeps ulps of 1.
+//   A target on a source, or within rounding of one, has a denominator of rounding
+//   where delta is 0, r about 1e16, and r G R x_k would leave a rounding as large as G
+//   although the pair's velocity is 0. So where a class has delta^2 below kCareD, pairs
+//   with a denominator below kCareD are left out of the sums and added as
+//   r G (R x_k - R x_i), which is 0 for equal points: their offsets are equal bit for
+//   bit. Only source tiles with a source as near to c as the targets can hold such a
+//   pair. Those track their largest reciprocal, one integer instruction a pair, and
+//   are summed again, with comparisons, if it is that large. This is a kernel of its own
+//   (CARE), so that other launches stay as they are. Its source loop is unrolled by 4,
+//   by 2 the level-5 Voronoi step takes 0.585 ms instead of 0.561. Without and with it, all
+//   classes with delta 0: level-5 Voronoi step 0.559 and 0.561 ms, level-5 vertex sum
+//   241.8 and 243.5 us, ten level-4 steps 2.01 and 2.10 ms.
 // * wide form (13 operations), for targets all over the sphere: the fused
 //   1 - x.y + delta^2 of the global coordinates and sum_k w (x_k - x_i).
 //   STRICT variants always take it, with the denominator rounded like the
@@ -161,6 +180,17 @@ __device__ __forceinline__ double frame_dot(const double* e, double vx, double v
 // ---------------------------------------------------------------------------
 constexpr float kFrameRho2 = 0.72f;  // frame form: |t|^2 at most (|t| <= 0.85)
 constexpr int kOwnTiles = 2048;     // bits of the own-tile map
+// r at most 1e6, and the rounding of r G R x_k at most 1e-10 G
+constexpr double kCareD = 1.0 / (1 << 20);
+
+constexpr int kCareHi = 0x3eb00000;  // high word of kCareD
+// high word from which a reciprocal's seed (relative error below 1e-6) may be that of a
+// denominator below kCareD: 1/kCareD's, less 2^-19 of it
+constexpr unsigned kMostHi = 0x41300000 - 4;
+
+__device__ __forceinline__ bool tiny_denominator(double D) {
+  return (__double2hiint(D) & 0x7fffffff) < kCareHi;  // |D| < kCareD
+}
 
 template <int NT, int TPT, int TS>
 struct Fp64Smem {
@@ -202,12 +232,20 @@ __device__ __forceinline__ double wide_denominator(double qx, double qy, double 
   return __dadd_rn(__dsub_rn(1.0, s), d2);
 }
 
-// Source j of the staged tile (index k) against the thread's targets. MASK: skip
-// the self pair, needed only in tiles that may hold the CTA's own points.
-template <int TPT, bool FRAME, bool STRICT, bool MASK, class Smem>
+// Source j of the staged tile (index k) against the thread's targets. HOW: kSelf skips
+// the self pair, needed only in tiles that may hold the CTA's own points; in the frame form
+// kTiny skips pairs with a tiny denominator and kMost takes down the high word of the
+// largest reciprocal of the others (a negative one counts as larger than any).
+enum { kSelf = 1, kTiny = 2, kMost = 4 };
+template <int HOW>
+struct How {
+  static constexpr int value = HOW;
+};
+
+template <int TPT, bool FRAME, bool STRICT, int HOW, class Smem>
 __device__ __forceinline__ void fp64_source(const Smem& sm, int j, int k, const double (*tg)[4],
                                             const int* self_k, double d2, double one_plus_d2,
-                                            double (*f)[3]) {
+                                            double (*f)[3], unsigned& most) {
   const double2 a = sm.a[j], b = sm.b[j];
   double2 c = make_double2(0.0, 0.0);
   if (FRAME) c = sm.c[j];
@@ -217,15 +255,19 @@ __device__ __forceinline__ void fp64_source(const Smem& sm, int j, int k, const 
       double D = fma(b.x, tg[t][2], tg[t][3]);
       D = fma(a.x, tg[t][0], D);
       D = fma(a.y, tg[t][1], D);
-      double r = rcp_f64(D);
-      if (MASK) r = (k == self_k[t]) ? 0.0 : r;
+      // the seed's low word is 0, and from a seed of 0 the reciprocal comes out as 0
+      const bool skip = ((HOW & kSelf) && k == self_k[t]) || ((HOW & kTiny) && tiny_denominator(D));
+      double r = rcp_seed_f64(D);
+      if (HOW & (kSelf | kTiny)) r = __hiloint2double(skip ? 0 : __double2hiint(r), 0);
+      if (HOW & kMost) most = max(most, (unsigned)__double2hiint(r));
+      r = rcp_refine_f64(D, r);
       f[t][0] = fma(r, b.y, f[t][0]);
       f[t][1] = fma(r, c.x, f[t][1]);
       f[t][2] = fma(r, c.y, f[t][2]);
     } else {
       const double D = wide_denominator<STRICT>(a.x, a.y, b.x, tg[t], d2, one_plus_d2);
       double w = __dmul_rn(b.y, rcp_f64(D));
-      if (MASK) w = (k == self_k[t]) ? 0.0 : w;
+      if (HOW & kSelf) w = (k == self_k[t]) ? 0.0 : w;
       f[t][0] = fma(w, a.x - tg[t][0], f[t][0]);
       f[t][1] = fma(w, a.y - tg[t][1], f[t][1]);
       f[t][2] = fma(w, b.x - tg[t][2], f[t][2]);
@@ -233,13 +275,47 @@ __device__ __forceinline__ void fp64_source(const Smem& sm, int j, int k, const 
   }
 }
 
+// The pairs that kTiny left out of the tile at ts (sources up to end): as differences
+// in the frame. Points with equal offsets are one point, whose denominator is taken as
+// the wide form has it: the pair is 0, or NaN where 1 - x.x + delta^2 rounds to 0.
+template <int TPT, class Smem>
+__device__ __forceinline__ void fp64_tiny_pairs(const Smem& sm, const double4* src, int ts, int end,
+                                                const double (*tg)[4], const int* self_k,
+                                                double one_plus_d2, double (*f)[3],
+                                                const UnitBounds& ub) {
+#pragma unroll 1
+  for (int j = 0; j < end - ts; ++j) {
+    const double2 a = sm.a[j];
+    const double ak = sm.b[j].x;
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) {
+      double D = fma(ak, tg[t][2], tg[t][3]);
+      D = fma(a.x, tg[t][0], D);
+      D = fma(a.y, tg[t][1], D);
+      if (!tiny_denominator(D) || ts + j == self_k[t]) continue;
+      if (!TC_BC(ub.rec, BC_PAIR_SRC, ts + j, ub.src_len)) continue;
+      const double4 q = src[ts + j];
+      const double x[3] = {q.x, q.y, q.z};
+      const double d[3] = {a.x + tg[t][0], a.y + tg[t][1], (1.0 - ak) - tg[t][2]};
+      if (d[0] == 0.0 && d[1] == 0.0 && d[2] == 0.0)
+        D = wide_denominator<false>(q.x, q.y, q.z, x, 0.0, one_plus_d2);
+      const double w = __dmul_rn(q.w, rcp_f64(D));
+#pragma unroll
+      for (int c = 0; c < 3; ++c) f[t][c] = fma(w, d[c], f[t][c]);
+    }
+  }
+}
+
 // Sources [c0, c1) against the thread's targets, totals in sm.acc. SHORT: the last
 // tile is staged and walked to its end only (a chunk need not be whole tiles);
-// otherwise it is padded, and the loop's length is known when it is compiled.
-template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool FRAME, bool STRICT, class Smem>
+// otherwise it is padded, and the loop's length is known when it is compiled. CARE
+// (frame form): source tiles with |s|^2 <= near2 are looked through for tiny
+// denominators, and count as own tiles.
+template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool FRAME, bool CARE, bool STRICT,
+          class Smem>
 __device__ __forceinline__ void fp64_sum(const double4* __restrict__ src, int c0, int c1, Smem& sm,
                                          const double (*tg)[4], const int* self_k, bool idle,
-                                         double d2, const UnitBounds& ub) {
+                                         double d2, double near2, const UnitBounds& ub) {
   const double one_plus_d2 = 1.0 + d2;
   double f[TPT][3];
 #pragma unroll
@@ -247,6 +323,9 @@ __device__ __forceinline__ void fp64_sum(const double4* __restrict__ src, int c0
   for (int ts = c0; ts < c1; ts += TS) {
     __syncthreads();
     const int len = SHORT ? min(TS, (c1 - ts + UNROLL - 1) / UNROLL * UNROLL) : TS;
+    const int tile = (ts - c0) / TS % kOwnTiles;
+    unsigned most = 0;
+    bool near = false;
     for (int j = threadIdx.x; j < len; j += NT) {
       const int k = ts + j;
       // padding: zero weight and (frame) a denominator of at least 1 off the targets
@@ -261,22 +340,34 @@ __device__ __forceinline__ void fp64_sum(const double4* __restrict__ src, int c0
         sm.a[j] = in ? make_double2(s1, s2) : make_double2(0.0, 0.0);
         sm.b[j] = in ? make_double2(ak, __dmul_rn(q.w, s1)) : make_double2(1.0, 0.0);
         sm.c[j] = in ? make_double2(__dmul_rn(q.w, s2), fma(-q.w, ak, q.w)) : make_double2(0.0, 0.0);
+        if (CARE) near |= in && fma(dx, dx, fma(dy, dy, dz * dz)) <= near2;
       } else {
         sm.a[j] = make_double2(q.x, q.y);
         sm.b[j] = make_double2(q.z, q.w);
       }
     }
+    if (CARE && near) atomicOr(&sm.own[tile / 32], 1u << (tile % 32));
     __syncthreads();
     if (idle) continue;  // a warp past the last target only stages
-    const int tile = (ts - c0) / TS % kOwnTiles;
-    if ((sm.own[tile / 32] >> (tile % 32)) & 1u) {
-#pragma unroll UNROLL
-      for (int j = 0; j < len; ++j)
-        fp64_source<TPT, FRAME, STRICT, true>(sm, j, ts + j, tg, self_k, d2, one_plus_d2, f);
+    const bool own = (sm.own[tile / 32] >> (tile % 32)) & 1u;
+    auto sum = [&](auto how, int n) {
+#pragma unroll (CARE ? 4 : UNROLL)
+      for (int j = 0; j < n; ++j)
+        fp64_source<TPT, FRAME, STRICT, decltype(how)::value>(sm, j, ts + j, tg, self_k, d2,
+                                                              one_plus_d2, f, most);
+    };
+    if (own) {
+      sum(How<CARE ? kSelf | kMost : kSelf>{}, len);
+      if (CARE && most >= kMostHi) {
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) f[t][0] = f[t][1] = f[t][2] = 0.0;
+#pragma unroll 1
+        for (int j = 0; j < len; ++j)
+          fp64_source<TPT, FRAME, STRICT, kSelf | kTiny>(sm, j, ts + j, tg, self_k, d2, one_plus_d2, f, most);
+        fp64_tiny_pairs<TPT>(sm, src, ts, min(c1, ts + TS), tg, self_k, one_plus_d2, f, ub);
+      }
     } else {
-#pragma unroll UNROLL
-      for (int j = 0; j < len; ++j)
-        fp64_source<TPT, FRAME, STRICT, false>(sm, j, ts + j, tg, self_k, d2, one_plus_d2, f);
+      sum(How<0>{}, len);
     }
 #pragma unroll
     for (int t = 0; t < TPT; ++t)
@@ -292,7 +383,7 @@ __device__ __forceinline__ void fp64_sum(const double4* __restrict__ src, int c0
 // i_end)) against the sources [c0, c1); FP64 sums written to out[pos],
 // out[stride + pos], out[2*stride + pos]. A target whose index is i has the
 // source index i + self_offset and skips itself (self_offset != kNoSelf).
-template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool STRICT>
+template <int NT, int TPT, int TS, int UNROLL, bool SHORT, bool STRICT, bool CARE>
 __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const int* __restrict__ perm,
                                           int tile0, int i_end, int self_offset, double d2,
                                           bool compact, const double4* __restrict__ src, int c0,
@@ -315,7 +406,7 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
     const bool okx = TC_BC(ub.rec, BC_PAIR_X, ld, ub.x_len);
 #pragma unroll
     for (int c = 0; c < 3; ++c) xi[t][c] = okx ? x[3 * (size_t)ld + c] : 0.0;
-    self_k[t] = has_self && valid ? ld + self_offset : -1;
+    self_k[t] = has_self ? ld + self_offset : -1;
     // points far off the sphere (or not finite) have no say in the origin
     const double n2 = fma(xi[t][0], xi[t][0], fma(xi[t][1], xi[t][1], xi[t][2] * xi[t][2]));
     if (!STRICT && compact && valid && n2 > 0.25 && n2 < 4.0) {
@@ -352,6 +443,7 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
       atomicOr(&sm.own[tile / 32], 1u << (tile % 32));
     }
   bool frame = false;
+  double near2 = -1.0;
   double tg[TPT][4];  // frame: -t_1, -t_2, 1 - b_i, b_i'; wide: x, y, z
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {
@@ -403,6 +495,8 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
 #pragma unroll
       for (int w = 0; w < NT / 32; ++w) r = max(r, sm.rho[w]);
       frame = __uint_as_float(r) <= kFrameRho2;
+      // a denominator below kCareD: |s| <= |t| + 0.0015, (|t| + 0.0015)^2 <= 1.05 |t|^2 + 5e-5
+      if (CARE && d2 < kCareD) near2 = 1.05 * (double)__uint_as_float(r) + 5e-5;
       if (!frame) {
 #pragma unroll
         for (int t = 0; t < TPT; ++t) {
@@ -415,9 +509,11 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
   }
   const bool idle = tile0 + warp * 32 >= i_end;
   if (frame)
-    fp64_sum<NT, TPT, TS, UNROLL, SHORT, true, false>(src, c0, c1, sm, tg, self_k, idle, d2, ub);
+    fp64_sum<NT, TPT, TS, UNROLL, SHORT, true, CARE, false>(src, c0, c1, sm, tg, self_k, idle, d2,
+                                                            near2, ub);
   else
-    fp64_sum<NT, TPT, TS, 2, SHORT, false, STRICT>(src, c0, c1, sm, tg, self_k, idle, d2, ub);
+    fp64_sum<NT, TPT, TS, 2, SHORT, false, false, STRICT>(src, c0, c1, sm, tg, self_k, idle, d2, 0.0,
+                                                          ub);
 #pragma unroll
   for (int t = 0; t < TPT; ++t) {
     const int i = tile0 + (int)threadIdx.x + t * NT;
@@ -444,7 +540,7 @@ __device__ __forceinline__ void fp64_unit(const double* __restrict__ x, const in
   }
 }
 
-template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
+template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT, bool CARE>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P) {
   chain_begin();
   __shared__ Fp64Smem<NT, TPT, TS> sm;
@@ -456,7 +552,7 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P)
   const long long base = (long long)blockIdx.y * 3 * (long long)stride + G.out_offset;
   double* out = P.partial + base;
   const UnitBounds ub{P.bc, G.x_len, G.perm_len, P.src_len, base, P.partial_len};
-  fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT>(
+  fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT, CARE>(
       G.x, G.perm, tile0, G.i1, G.self_offset, G.d2, G.compact != 0, P.src, c0, c1, out, stride, sm,
       ub);
 }
@@ -1042,6 +1138,7 @@ struct BatchLaunch {
   const double4* src;
   double* partial;   // partial[(chunk*3 + c)*stride + row]
   size_t stride;
+  bool care;              // FP64: a segment has d2 < kCareD
   BoundsRec* bc;          // checked build: violation record (null: release build)
   int n_segs;             // checked build: entries in segs
   long long src_len;      // checked build: packed sources in src
@@ -1073,7 +1170,7 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp32c_batch_kernel(const BatchL
   }
 }
 
-template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT>
+template <int NT, int TPT, int TS, int MINB, int UNROLL, bool SHORT, bool STRICT, bool CARE>
 __global__ void __launch_bounds__(NT, MINB) pair_fp64_batch_kernel(const BatchLaunch B) {
   chain_begin();
   __shared__ Fp64Smem<NT, TPT, TS> sm;
@@ -1085,7 +1182,7 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_batch_kernel(const BatchLa
     const long long base = (long long)I.chunk * 3 * (long long)B.stride + S.out_offset;
     double* out = B.partial + base;
     const UnitBounds ub{B.bc, S.x_len, S.perm_len, B.src_len, base, B.partial_len};
-    fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT>(
+    fp64_unit<NT, TPT, TS, UNROLL, SHORT, STRICT, CARE>(
         S.x, S.perm, I.tile0, I.i1, S.self_offset, S.d2, S.compact != 0, B.src, I.c0, I.c1, out,
         B.stride, sm, ub);
   }

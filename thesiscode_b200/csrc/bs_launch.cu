@@ -43,11 +43,17 @@ constexpr int kTS = 256;
 
 template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64(dim3 g, cudaStream_t s, const PairLaunch& P) {
-  launch_chained(pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, dim3(g), dim3(NT), 0, s, P);
+  const auto kernel = !STRICT && P.care
+                          ? pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, !STRICT>
+                          : pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, false>;
+  launch_chained(kernel, dim3(g), dim3(NT), 0, s, P);
 }
 template <int NT, int TPT, int MINB, int UNROLL, bool SHORT, bool STRICT>
 void launch64b(int g, cudaStream_t s, const BatchLaunch& B) {
-  launch_chained(pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, dim3(g), dim3(NT), 0, s, B);
+  const auto kernel = !STRICT && B.care
+                          ? pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, !STRICT>
+                          : pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, false>;
+  launch_chained(kernel, dim3(g), dim3(NT), 0, s, B);
 }
 template <int NT, int T, int TS, int FLUSH, int MINB, int UNROLL, int FM>
 void launch32b(int g, cudaStream_t s, const BatchLaunch& B) {
@@ -61,9 +67,9 @@ void launch32(dim3 g, cudaStream_t s, const PairLaunch& P) {
 #define V64(NT, TPT, MINB, UNROLL, SHORT, STRICT)                                            \
   PairVariant { TC_FP64, NT, TPT, kTS, !STRICT, MINB, UNROLL,                                 \
                 launch64<NT, TPT, MINB, UNROLL, SHORT, STRICT>,                               \
-                (const void*)pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>,     \
+                (const void*)pair_fp64_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, false>,     \
                 launch64b<NT, TPT, MINB, UNROLL, SHORT, STRICT>,                              \
-                (const void*)pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT>, 0 }
+                (const void*)pair_fp64_batch_kernel<NT, TPT, kTS, MINB, UNROLL, SHORT, STRICT, false>, 0 }
 // FP32C: T targets per thread, source tiles of TS, FP32 flush every FLUSH sources,
 // form bits FM
 #define V32T(NT, T, TS, FLUSH, MINB, UNROLL, FM)                                         \
@@ -317,6 +323,7 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
     g.self_offset = segs[s].self_offset;
     g.d2 = segs[s].d2;
     g.compact = len >= kCompactTiles * tb;
+    P->care = P->care || (g.compact && g.d2 < kCareD);
     g.x_len = bc_extent(ctx, BC_PAIR_X, segs[s].x_len);
     g.perm_len = bc_extent(ctx, BC_PAIR_PERM, segs[s].perm_len);
     g.tile_begin = tiles;
