@@ -468,8 +468,8 @@ __device__ __forceinline__ void adj_next(const AdjNext& N, size_t j, double g) {
 // of it: three launches a stage less, level 5 0.755 -> 0.731 ms a product, level 4
 // 0.118 -> 0.092.
 __global__ void __launch_bounds__(256) adj_combine_row_kernel(
-    const double* __restrict__ x, const double* __restrict__ ut, const double* __restrict__ zeta,
-    const double* __restrict__ area, int n, const double* __restrict__ p, int chunks,
+    const double* x, const double* ut, const double* zeta, const double* area, int n,
+    const double* p, int chunks,
     const AdjNext next, BoundsRec* bc, long long p_len) {
   chain_begin();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -508,13 +508,11 @@ __global__ void __launch_bounds__(256) adj_combine_row_kernel(
 // v_i = ut_i x x_i with ut_i = mu_x,i + (-2 Omega mu_z,i) z_hat, mu = dt * l_k.
 // ROW: the row pass's inputs only (ra, rb, rc); otherwise the other passes' as well.
 template <bool ROW>
-__global__ void adj_prepare_kernel(const double* __restrict__ x, const double* __restrict__ lkx,
-                                   const double* __restrict__ lkz, const double* __restrict__ zeta,
-                                   const double* __restrict__ area, int n, double dt, double m2omega,
-                                   double* __restrict__ ut, double* __restrict__ v,
-                                   double4* __restrict__ src1, double4* __restrict__ src2a,
-                                   double2* __restrict__ src2b, double4* __restrict__ ra,
-                                   double4* __restrict__ rb, double* __restrict__ rc) {
+__global__ void adj_prepare_kernel(const double* x, const double* lkx, const double* lkz,
+                                   const double* zeta, const double* area, int n, double dt,
+                                   double m2omega, double* ut, double* v, double4* src1,
+                                   double4* src2a, double2* src2b, double4* ra, double4* rb,
+                                   double* rc) {
   chain_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -569,8 +567,7 @@ __global__ void adj_combine_kernel(const double* __restrict__ x, const double* _
 }
 
 // Start of a step's backward sweep: acc = l' (the identity part), lk_4 = b l'.
-__global__ void adj_begin_kernel(const double* __restrict__ lam, double b, double* __restrict__ acc,
-                                 double* __restrict__ lk, size_t n) {
+__global__ void adj_begin_kernel(const double* lam, double b, double* acc, double* lk, size_t n) {
   chain_begin();
   size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (j >= n) return;

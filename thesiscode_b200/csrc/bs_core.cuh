@@ -23,7 +23,10 @@ namespace tcb {
 constexpr int kNoSelf = INT32_MIN;
 
 // Start of a kernel launched by launch_chained: everything before it in the stream is
-// done when this returns, and the next chained kernel may be set up meanwhile.
+// done when this returns, and the next chained kernel may be set up meanwhile. The kernel's
+// lifetime overlaps its predecessor's, so its parameters carry no __restrict__ on what a
+// predecessor may write: that would promise that nothing else writes it while the kernel
+// runs, and allow loads that do not see it. Functions called after this may have it.
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

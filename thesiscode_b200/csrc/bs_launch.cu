@@ -426,8 +426,8 @@ struct PackBounds {
   long long in_len, out_len;
 };
 
-__global__ void pack_kernel(const double* __restrict__ x, const double* __restrict__ zeta,
-                            const double* __restrict__ area, int n, double4* __restrict__ out,
+__global__ void pack_kernel(const double* x, const double* zeta, const double* area, int n,
+                            double4* out,
                             const PackBounds pb) {
   chain_begin();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -440,9 +440,8 @@ __global__ void pack_kernel(const double* __restrict__ x, const double* __restri
 
 // Forced model: stage-1 sources from the absolute vorticity at time t; the
 // relative vorticity is also written to z0 (it is the state's zeta at t).
-__global__ void pack_strat_kernel(const double* __restrict__ x, const double* __restrict__ absv,
-                                  const double* __restrict__ area, int n, double two_omega,
-                                  double t, double* __restrict__ zeta, double4* __restrict__ out,
+__global__ void pack_strat_kernel(const double* x, const double* absv, const double* area, int n,
+                                  double two_omega, double t, double* zeta, double4* out,
                                   const PackBounds pb) {
   chain_begin();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -540,7 +539,7 @@ __device__ __forceinline__ int epilogue_row(int* first) {
 // every lane's); the checked build checks each read against partial_len doubles
 // (site: BC_EPI_PARTIAL or BC_STAGE_PARTIAL).
 template <bool SPLIT>
-__device__ __forceinline__ void reduce_row(const double* __restrict__ partial, int first,
+__device__ __forceinline__ void reduce_row(const double* partial, int first,
                                            int nchunks, size_t n_out, size_t row, double T[3],
                                            BoundsRec* rec, int site, long long partial_len) {
   T[0] = T[1] = T[2] = 0.0;
@@ -578,11 +577,10 @@ struct EpiBounds {
 };
 
 template <bool SPLIT>
-__global__ void __launch_bounds__(kEpiThreads) velocity_epilogue_kernel(const double* __restrict__ x, const int* __restrict__ perm,
+__global__ void __launch_bounds__(kEpiThreads) velocity_epilogue_kernel(const double* x, const int* perm,
                                          int m, int i0, int i1, int row_offset, int n_out,
-                                         int nchunks, const double* __restrict__ partial,
-                                         double m2omega, double* __restrict__ dX,
-                                         double* __restrict__ dVort, const EpiBounds eb) {
+                                         int nchunks, const double* partial,
+                                         double m2omega, double* dX, double* dVort, const EpiBounds eb) {
   chain_begin();
   int first;
   const int p = epilogue_row<SPLIT>(&first);
@@ -772,8 +770,7 @@ __global__ void __launch_bounds__(kEpiThreads) stage_epilogue_kernel(const Stage
   }
 }
 
-__global__ void ke_finalize_kernel(const double* __restrict__ blocks, int nblocks,
-                                   double* __restrict__ out) {
+__global__ void ke_finalize_kernel(const double* blocks, int nblocks, double* out) {
   chain_begin();
   __shared__ double red[256];
   double s = 0.0;
