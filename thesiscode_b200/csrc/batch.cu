@@ -192,7 +192,7 @@ int upload_segments(tc_ctx* ctx, tc_batch_plan& B) {
       g.out_offset = cls == 0 ? 0 : B.nA_tot;
       g.self_offset = cls == 0 ? 0 : tcb::kNoSelf;
       g.d2 = ctx->delta[cls] * ctx->delta[cls];
-      g.compact = 1;
+      g.targets = cls == 0 ? B.nA[b] : B.nV[b];
       g.perm_len = g.perm ? (long long)((cls == 0 ? R.permA : R.permV).bytes / sizeof(int)) : 0;
       g.x = cls == 0 ? R.x0A.as<double>() : R.x0V.as<double>();
       g.x_len = (long long)((cls == 0 ? R.x0A : R.x0V).bytes / (3 * sizeof(double)));
@@ -432,7 +432,8 @@ static int batch_rk4_impl(tc_ctx* ctx, int count, const int* nA, const int* nV, 
   // tc_set_pair_variant
   const bool fp64 = ctx->precision == TC_FP64, tune = (flags & TC_BATCH_AUTOTUNE) != 0;
   const bool fixed = !(fp64 ? ctx->auto64 : ctx->auto32);
-  const int plain = fp64 ? (ctx->auto64 ? tcb::kAuto64Default : ctx->var64) : ctx->var32;
+  const int plain = tcb::batch_variant(ctx, *std::max_element(B.nA.begin(), B.nA.end()),
+                                       (long long)B.nA_tot + B.nV_tot);
   if (B.variant < 0 || (tune && !B.tuned) || (!tune && fixed && B.variant != plain)) {
     if ((rc = tune ? autotune(ctx, B) : build_items(ctx, B, plain, 4096))) {
       B.variant = -1;

@@ -153,11 +153,13 @@ int select_variant(tc_ctx* ctx, int precision, int id) {
 constexpr int kAutoFewSources = 12288, kAutoMidSources = 131072;
 constexpr int kAutoFewVariant = 1, kAutoMidVariant = 12, kAutoLargeVariant = 0;
 
+static int auto32_variant(int n) {
+  return n < kAutoFewSources ? kAutoFewVariant : n < kAutoMidSources ? kAutoMidVariant : kAutoLargeVariant;
+}
+
 int use_fp32c_variant(tc_ctx* ctx, int n) {
   if (!ctx->auto32) return TC_OK;
-  const int want = n < kAutoFewSources   ? kAutoFewVariant
-                   : n < kAutoMidSources ? kAutoMidVariant
-                                         : kAutoLargeVariant;
+  const int want = auto32_variant(n);
   return want == ctx->var32 ? TC_OK : select_variant(ctx, TC_FP32C, want);
 }
 
@@ -280,16 +282,16 @@ static int chunk_length(const tc_ctx* ctx, const PairCfg& cfg, int slots, int ti
 constexpr int kFewSources = 12288, kMidSources = 65536;
 constexpr int kFewTargets = 6144, kMidTargets = 24576;
 
-static int auto64_variant(const SegDesc* segs, int nseg, int n) {
-  const int targets = count_tiles(segs, nseg, 1);
+static int auto64_variant(long long targets, int n) {
   if (n < kFewSources || targets < kFewTargets) return kAuto64Small;
   return n < kMidSources || targets < kMidTargets ? kAuto64Mid : kAuto64Default;
 }
 
-// A tile of 1/16 of the sphere's targets has a radius of 0.5 to 0.8, within the frame
-// form's limit; fewer tiles than that are not worth the search for a frame (level 3,
-// 1,280 panels: 21.6 us a sum with it, 19.6 without).
-constexpr int kCompactTiles = 16;
+int batch_variant(const tc_ctx* ctx, int largest, long long targets) {
+  if (ctx->precision == TC_FP64)
+    return ctx->auto64 ? auto64_variant(targets, largest) : ctx->var64;
+  return ctx->auto32 ? auto32_variant(largest) : ctx->var32;
+}
 
 // Tiles and chunking of one pair launch: the target segments, the grid and the
 // chunk length (partial sums need S * 3 * n_out doubles).
@@ -301,7 +303,7 @@ static int plan_pairs(tc_ctx* ctx, const SegDesc* segs, int nseg, const double4*
     if (rc0) return rc0;
   }
   if (fp64 && ctx->auto64 && n > 0 && count_tiles(segs, nseg, 1) > 0) {
-    const int want = auto64_variant(segs, nseg, n);
+    const int want = auto64_variant(count_tiles(segs, nseg, 1), n);
     if (want != ctx->var64) {
       const int rc = select_variant(ctx, TC_FP64, want);
       if (rc) return rc;

@@ -260,4 +260,7 @@ int variant_count(int precision);
 int select_variant(tc_ctx* ctx, int precision, int id);
 // With ctx->auto32, selects the FP32C variant for a launch over n sources.
 int use_fp32c_variant(tc_ctx* ctx, int n);
+// Variant of an ensemble whose launch shape is not tuned: the automatic one for the panels of
+// its largest member (and all members' targets, which fill the GPU together), or the one set.
+int batch_variant(const tc_ctx* ctx, int largest, long long targets);
 }  // namespace tcb
