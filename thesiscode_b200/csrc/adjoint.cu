@@ -828,13 +828,15 @@ int adjoint_impl(tc_ctx* ctx, const double* xA0, const double* zetaA0, const dou
   if ((rc = W.ck.ensure((size_t)ncheck * B)) || (rc = W.ys.ensure((size_t)ckpt_every * 4 * B)) ||
       (rc = W.lam.ensure(B)) || (rc = W.lk.ensure(B)) || (rc = W.tmp.ensure(B)) ||
       (rc = W.ut.ensure(3 * (size_t)nA * sizeof(double))) ||
-      (rc = W.v.ensure(3 * (size_t)nA * sizeof(double))) ||
-      (rc = W.s1.ensure((size_t)nA * sizeof(double4))) ||
-      (rc = W.s2a.ensure((size_t)nA * sizeof(double4))) ||
-      (rc = W.s2b.ensure((size_t)nA * sizeof(double2))) ||
       (rc = W.ra.ensure((size_t)nA * sizeof(double4))) ||
       (rc = W.rb.ensure((size_t)nA * sizeof(double4))) ||
       (rc = W.rc.ensure((size_t)nA * sizeof(double))))
+    return rc;
+  // inputs of the passes other than the row pass
+  if (ctx->adj_mode < 3 && ((rc = W.v.ensure(3 * (size_t)nA * sizeof(double))) ||
+                            (rc = W.s1.ensure((size_t)nA * sizeof(double4))) ||
+                            (rc = W.s2a.ensure((size_t)nA * sizeof(double4))) ||
+                            (rc = W.s2b.ensure((size_t)nA * sizeof(double2)))))
     return rc;
   double* ck = W.ck.as<double>();
   double* ys = W.ys.as<double>();

@@ -122,7 +122,7 @@ bool stage_ready(tc_ctx* ctx, size_t total) {
   }
   tcb::HostStage& S = ctx->stage;
   if (!S.host) {
-    if (S.plain < tcb::HostStage::kPlainFirst) {
+    if (S.refused || S.plain < tcb::HostStage::kPlainFirst) {
       ++S.plain;
       return false;
     }
@@ -132,6 +132,7 @@ bool stage_ready(tc_ctx* ctx, size_t total) {
         cudaEventCreateWithFlags(&S.read, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       if (h) cudaFreeHost(h);
+      S.refused = true;
       return false;  // no page-locked memory to be had: the arrays are copied one by one
     }
     S.host = static_cast<char*>(h);

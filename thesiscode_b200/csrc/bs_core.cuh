@@ -50,7 +50,8 @@ struct PairLaunch {
   int nseg;
   const double4* src;   // packed sources {x, y, z, G}
   int n;                // number of sources
-  int chunk_len;        // sources per blockIdx.y chunk (multiple of the tile)
+  int chunk_len;        // sources per blockIdx.y chunk (multiple of the tile; FP64 SHORT
+                        // shapes: of 16)
   double* partial;      // partial[(chunk*3 + c)*n_out + row]
   int n_out;
   bool care;            // FP64: a segment with frames has d2 < kCareD
@@ -632,8 +633,8 @@ __global__ void __launch_bounds__(NT, MINB) pair_fp64_kernel(const PairLaunch P)
 // Form bits (FM): bit 3 always set (the source-paired form; the bit value
 // is part of the variant-info ABI); bit 1 keeps the FP64 accumulators in
 // shared memory (one slot per thread, target and coordinate: 6 fewer
-// registers per target); bit 2 gives near tiles hi/lo offsets; bits 8-9 hold
-// log2 FARK.
+// registers per target); bit 2 gives near tiles hi/lo offsets; bit 4 lets two targets
+// share reciprocals in every second far source pair; bits 8-9 hold log2 FARK.
 // HILO (bit 2): near tiles take d = s - t from hi/lo FP32 splits of both
 // offsets, (s_hi - t_hi) + (s_lo - t_lo): the rounding of the offsets to FP32
 // (an absolute error of ulps of the patch radius, the dominant FP32C error

@@ -167,10 +167,6 @@ int resolve_slots(tc_ctx* ctx) {
   cudaDeviceProp prop;
   TC_CUDA_TRY(cudaGetDeviceProperties(&prop, ctx->device));
   ctx->num_sms = prop.multiProcessorCount;
-  int blocks = 0;
-  TC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &blocks, kVariants64[kAuto64Default].fn, kVariants64[kAuto64Default].nt, 0));
-  ctx->slots64_default = std::max(1, blocks) * ctx->num_sms;
   int rc = select_variant(ctx, TC_FP64, ctx->var64);
   if (rc) return rc;
   return select_variant(ctx, TC_FP32C, ctx->var32);
@@ -178,7 +174,7 @@ int resolve_slots(tc_ctx* ctx) {
 
 // Number of source chunks: the split that best fills the resident CTA slots
 // (waves of tiles x chunks), never cutting chunks below ctx->min_chunk.
-static int choose_chunks(int tiles, int n, int ts, int slots, int min_chunk, int max_chunks) {
+static int choose_chunks(int tiles, int n, int slots, int min_chunk, int max_chunks) {
   int best = 1;
   double best_eff = 0.0;
   for (int s = 1; s <= max_chunks; ++s) {
@@ -193,7 +189,6 @@ static int choose_chunks(int tiles, int n, int ts, int slots, int min_chunk, int
     }
     if (eff > 0.97) break;
   }
-  (void)ts;
   return best;
 }
 
@@ -229,7 +224,7 @@ static int fine_chunk_len(int tiles, int n, int num_sms, int slots, int warps, i
 
 // Chunk length of whole-tile chunks (tiles of ts sources).
 static int whole_chunk_len(int tiles, int n, int ts, int slots, int min_chunk, int max_chunks) {
-  const int S = choose_chunks(tiles, n, ts, slots, min_chunk, max_chunks);
+  const int S = choose_chunks(tiles, n, slots, min_chunk, max_chunks);
   const int len = (n + S - 1) / S;
   return (len + ts - 1) / ts * ts;
 }

@@ -93,6 +93,7 @@ struct HostStage {
   static constexpr size_t kStageBytes = size_t(512) << 10;
   static constexpr int kPlainFirst = 16;  // transfers, 40 to 80 us saved by each pair of them
   int plain = 0;                          // copied array by array so far
+  bool refused = false;                   // the driver had none: not asked again
   char* host = nullptr;
   char* dev = nullptr;         // the same memory, as the GPU sees it
   cudaEvent_t read = nullptr;  // the last kernel that reads or writes the buffer
@@ -147,7 +148,6 @@ struct tc_ctx {
   int var64 = 2, var32 = 0;  // pair-kernel variants in use (see kVariants64/32)
   bool auto32 = true;  // FP32C variant chosen per launch by problem size (tc_set_pair_variant turns it off)
   bool auto64 = true;  // FP64 variant chosen per launch by its size (likewise)
-  int slots64_default = 0;  // resident CTAs per GPU of the default FP64 variant
   int target_order = TC_ORDER_HILBERT;  // visiting order of targets
   double adj_ms[3] = {0.0, 0.0, 0.0};  // last adjoint: forward sweep, recompute, backward
   int adj_mode = 6;  // adjoint VJP: 3-6 row pass, 0 two passes, 1 and 2 fused (tc_set_adjoint_mode)
