@@ -77,15 +77,17 @@ __global__ void small_keys_kernel(const SmallOrders P) {
                   : 0u;
 }
 
-// Exclusive prefix sum, over the CTA's threads in order, of eight counts each.
+// Exclusive prefix sum, over the CTA's threads in order, of eight counts each; the
+// thread's largest count.
 constexpr int kPer = kOrderCells / kOrderThreads;
-__device__ __forceinline__ void order_prefix(int* mine, int* wsum) {
+__device__ __forceinline__ int order_prefix(int* mine, int* wsum) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int n[kPer], total = 0;
+  int n[kPer], total = 0, most = 0;
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
     n[q] = mine[q];
     total += n[q];
+    most = max(most, n[q]);
   }
   int incl = total;
 #pragma unroll
@@ -102,6 +104,7 @@ __device__ __forceinline__ void order_prefix(int* mine, int* wsum) {
     mine[q] = base;
     base += n[q];
   }
+  return most;
 }
 
 // The order of n keys by a stable counting sort of idx, 8 key bits at a time, the lowest
@@ -110,7 +113,7 @@ __device__ __forceinline__ void order_prefix(int* mine, int* wsum) {
 // and counts digits as it goes, so a point's rank among its warp's points of that digit
 // is known at once; the counts' prefix sum, digits before warps, gives every point its
 // place.
-__device__ __forceinline__ void order_by_digits(const SmallOrder& S, const unsigned* keys,
+__device__ __noinline__ void order_by_digits(const SmallOrder& S, const unsigned* keys,
                                                 unsigned short* idx, int* counts, int* wsum) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int(*count)[kOrderWarps + 1] = reinterpret_cast<int(*)[kOrderWarps + 1]>(counts);
@@ -185,15 +188,10 @@ __global__ void __launch_bounds__(kOrderThreads) small_order_kernel(const SmallO
     atomicAdd(&cell[k >> kOrderShift], 1);
   }
   __syncthreads();
-  bool full = false;
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) full |= cell[tid * kPer + q] > kFullCell;
-  if (__syncthreads_or(full)) {
+  if (__syncthreads_or(order_prefix(cell + tid * kPer, wsum) > kFullCell)) {
     order_by_digits(S, keys, slot, cell, wsum);
     return;
   }
-  order_prefix(cell + tid * kPer, wsum);
-  __syncthreads();
   for (int j = tid; j < S.n; j += kOrderThreads)
     slot[atomicAdd(&cell[keys[j] >> kOrderShift], 1)] = (unsigned short)j;
   __syncthreads();
