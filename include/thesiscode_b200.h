@@ -253,7 +253,9 @@ int tc_rk4_steps_done(tc_ctx* ctx, long long* steps);
  * adjoint of the step (exact gradient of the RK4 map), FP64, state
  * checkpointed every ckpt_every steps and stage inputs recomputed per
  * segment. Host arrays: xA0(3,nA), zetaA0, areaA in; J, g_zeta0(nA),
- * g_x0(3,nA) out. Replaces the context's loaded RK4 state. */
+ * g_x0(3,nA) out. Replaces the context's loaded RK4 state. The context keeps
+ * up to 512 MB of the adjoint's buffers for the next call, until tc_reset_rk4
+ * or tc_destroy. */
 int tc_rk4_adjoint(tc_ctx* ctx, const double* xA0, const double* zetaA0, const double* areaA,
                    int nA, double dt, int nsteps, int ckpt_every, int functional, int probe,
                    double* J, double* g_zeta0, double* g_x0);
@@ -328,16 +330,19 @@ int tc_device_count(int* count);
  * targets/CTA, form}. FP32C form: bit 3 = source-paired kernel (set in every
  * variant: the two lanes of each f32x2 instruction carry two sources of one
  * target), bit 1 = FP64 accumulators in shared memory, bit 2 = hi/lo
- * near-pair offsets (the accurate variants), bits 8-9 = log2 of the flush
- * lengths between flushes in tiles whose every source is far. FP64 form: 0. */
+ * near-pair offsets (the accurate variants), bit 4 = two targets share
+ * reciprocals in every second far source pair, bits 8-9 = log2 of the flush
+ * lengths between flushes in tiles whose every source is far. FP64 form: 0.
+ * A number names a shape of this build only; another build may number other
+ * shapes so. Select by what tc_pair_variant_info says. */
 int tc_pair_variant_count(int precision, int* count);
 int tc_pair_variant_info(int precision, int id, int* info8);
 /* Select a variant. By default the variant is chosen per launch by problem
- * size. For FP32C: variant 1 below 131,072 sources, 0 above. For FP64:
- * variant 2, or variant 6 (the same shape with 32-source tiles and chunks of
- * any multiple of 32 sources) for launches that would fill less than 90% of
- * one wave of CTAs with whole 256-source chunks. Selecting a variant turns
- * the automatic choice off; id = -1 turns it back on. tc_get_pair_variant
+ * size. For FP32C: variant 1 below 12,288 sources, 12 below 131,072, else 0.
+ * For FP64: variant 6 below 12,288 sources or 6,144 targets, 7 below 65,536
+ * sources or 24,576 targets, else 2. An ensemble that is not tuned takes the
+ * choice for its largest member's panels. Selecting a variant turns the
+ * automatic choice off; id = -1 turns it back on. tc_get_pair_variant
  * returns the variant in use (with the automatic choice: the one last
  * used). */
 int tc_set_pair_variant(tc_ctx* ctx, int precision, int id);

@@ -281,9 +281,10 @@ std::vector<uint64_t> graph_key(const tc_ctx* ctx, const tc_batch_plan& B, doubl
 
 // Time one stage-0 pair launch of each (variant, chunk) candidate; keep the best.
 // Candidate launch shapes: the default of each precision first, then the
-// shapes that were fastest on some workload of the level-7 sweep, all with the
-// default's accuracy (64-source FP32 flush; a 128-source flush is faster by
-// about 1% and raises the error by half).
+// shapes that were fastest on some workload of the level-7 sweep. All flush FP32 sums
+// every 64 sources in tiles with near sources, and every 64 to 256 in others. Each is timed
+// once, so two contexts may settle on different shapes: 24 members of levels 3 to 5,
+// four FP32C steps, took 29.6 and 34.5 ms in two contexts.
 const int kTune32[] = {0, 1, 2, 3, 4, 5, 6, 7, 12};
 const int kTune64[] = {2, 0, 1, 3, 6, 7};
 

@@ -171,16 +171,21 @@ __device__ __forceinline__ double frame_dot(const double* e, double vx, double v
 //   operations).
 //
 // Either way the sums of at most a tile's 256 sources are added to totals in shared
-// memory: in one long chain the sums' rounding would outweigh the terms'. Against
-// an extended-precision sum (levels 3-6, three fields, delta 0 and 0.01) the frame
-// form at |t| <= 0.7 has 0.1 to 1.0 times the error of the plain sum
-// sum_k w (x_k - x_i), and 1 to 2 times at |t| up to 2, hence the limit.
+// memory: in one long chain the sums' rounding would outweigh the terms'. The frame
+// form's error grows with |t|, by which its largest sum, about sum r G along c, enters
+// u. Restated on the CPU with the same fused operations (level-5 panels and vertices, two
+// fields, delta 0 and 0.01, 12 frames), its rms error against 80-bit sums is this many
+// times that of the plain sum_k w (x_k - x_i): 0.3-0.9 at |t| 0.2, 0.8-1.0 at 0.4, 1.3-3
+// at 0.6, 2-6 at 0.85, where it is at most 8e-15 of the largest velocity. The limit is
+// where tiles of 1/16 of the sphere's targets still pass; most tiles have |t| of 0.1 to
+// 0.5, and whole runs are as far from 64-bit ones as with the plain sum (ten level-4
+// steps 2.6e-14 both, level-5 vertex sum 3.5e-14 and 3.8e-14, level 6 2.3e-14 both).
 //
 // Level 6 refined, 108,923 sources and 199,823 targets in three classes: 1.115e12
 // pairs/s with the wide form alone, at 14 operations, and now 1.53e12. 9 DFMA at
-// their nominal 2 cycles would allow 18.5e12 / 9 = 2.05e12; with the register reads
-// of a loop that shares a source among the targets (2.3 to 2.5 cycles) the bare loop
-// reaches 1.6e12.
+// their nominal 2 cycles would allow 18.5e12 / 9 = 2.05e12; the register reads of a
+// loop that shares a source among the targets make that 2.3 to 2.5 cycles. Level 8
+// reaches 1.60e12.
 // ---------------------------------------------------------------------------
 constexpr float kFrameRho2 = 0.72f;  // frame form: |t|^2 at most (|t| <= 0.85)
 // A tile of 1/16 of the sphere's targets has a radius of 0.5 to 0.8, within that limit;

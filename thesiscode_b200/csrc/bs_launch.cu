@@ -366,7 +366,8 @@ static int run_pairs(tc_ctx* ctx, const PairLaunch& P, dim3 grid) {
   return TC_OK;
 }
 
-// Chunks a launch may have: ctx->max_chunks, or for few rows up to kManyChunks as far as
+// Chunks a launch may have (24 bytes of partial sums a target each: 66 MB in a level-6
+// FP64 sum): ctx->max_chunks, or for few rows up to kManyChunks as far as
 // their partial sums stay small (a few hundred targets against many sources).
 static int most_chunks(const tc_ctx* ctx, int n_out) {
   constexpr size_t kManyChunks = 256, kManyBytes = size_t(64) << 20;
